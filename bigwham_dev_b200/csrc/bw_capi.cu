@@ -13,6 +13,7 @@
 #include "bigwham_b200.h"
 #include "bw_kernels.cuh"
 #include "bw_mm_kernels.cuh"
+#include "bw_multi_kernels.cuh"
 #include "bw_aca_kernels.cuh"
 #include "bw_assemble_kernels.cuh"
 #include "bw_devlayout_kernels.cuh"
@@ -67,6 +68,7 @@ struct DevPhase {
   int32_t *items = nullptr;        // chunk ranges of the items, in the order CTAs take them
   int *queue = nullptr;            // [next item, CTAs done], zero between launches
   bw::GatherSeg *gsegs = nullptr;  // phase 2: runs that fill G2
+  bw::RunRange *ranges = nullptr;  // phase 2: each chunk's runs (several right-hand sides), or null
   int64_t n_chunks = 0;
   int64_t n_items = 0;
   int64_t n_elems = 0;
@@ -110,6 +112,7 @@ struct bw_hmat {
   uint16_t *d_xt = nullptr, *d_t8 = nullptr;  // matmat operands (8x8 BF16 tiles, bw::kMmRhs columns)
   int32_t *d_perm0 = nullptr, *d_perm1 = nullptr;
   void *d_xp = nullptr, *d_t = nullptr, *d_g2 = nullptr;
+  void *d_xk = nullptr, *d_tk = nullptr;  // x and t of bw::kMultiMax right-hand sides, or null
   double *d_xh = nullptr, *d_yh = nullptr;
   double *h_xpin = nullptr, *h_ypin = nullptr;  // pinned staging of bw_matvec_host
   cudaEvent_t y_ready[4] = {nullptr, nullptr, nullptr, nullptr};  // bw_matvec_host: output pieces landed
@@ -176,6 +179,7 @@ struct bw_hmat {
           cudaFree(ph.items);
           cudaFree(ph.queue);
           cudaFree(ph.gsegs);
+          cudaFree(ph.ranges);
           ph = DevPhase{};
         }
     for (auto &o : dmm)
@@ -194,6 +198,8 @@ struct bw_hmat {
     cudaFree(d_xp);
     cudaFree(d_t);
     cudaFree(d_g2);
+    cudaFree(d_xk);
+    cudaFree(d_tk);
     cudaFree(d_xh);
     cudaFree(d_yh);
     if (h_xpin) cudaFreeHost(h_xpin);
@@ -211,6 +217,7 @@ struct bw_hmat {
     if (stream) cudaStreamDestroy(stream);
     d_perm0 = d_perm1 = nullptr;
     d_xp = d_t = d_g2 = nullptr;
+    d_xk = d_tk = nullptr;
     d_xh = d_yh = nullptr;
     d_err = nullptr;
     h_err = nullptr;
@@ -750,6 +757,110 @@ void launch_matmat_tc(bw_hmat *h, int o, const double *X, int64_t ldx, double *Y
   }
 }
 
+// Scratch and run tables of the FP64 / FP32 products with several right-hand
+// sides (bw_multi_kernels.cuh): 8 columns of x and t and 8 bytes per phase-2
+// chunk, about 1% of the block data.  Taken last; when they do not fit (the
+// device limit, or the device itself) such products apply one matvec per
+// column, as they do without these kernels.
+void alloc_multi(bw_hmat *h, int mask, bool with_t) {
+  const int64_t es = (mask & 1) ? 8 : 4, k = bw::kMultiMax;
+  if (!(mask & 3)) return;
+  std::vector<DevPhase *> made;
+  try {
+    for (int o = 0; o < (with_t ? 2 : 1); o++)
+      for (int p = 0; p < 2; p++) {
+        const bw::ChunkPlan &cp = h->op[o].ph[1].cp[p];
+        if (!(mask & (1 << p)) || cp.chunks.empty()) continue;
+        const auto rr = bw::run_ranges(cp);
+        static_assert(sizeof(rr[0]) == sizeof(bw::RunRange), "pairs of 32-bit integers");
+        DevPhase &dp = h->dev[o][p][1];
+        dp.ranges = static_cast<bw::RunRange *>(h->dmalloc(rr.size() * sizeof(bw::RunRange)));
+        made.push_back(&dp);
+        BW_CUDA(cudaMemcpy(dp.ranges, rr.data(), rr.size() * sizeof(bw::RunRange), cudaMemcpyHostToDevice));
+      }
+    h->d_xk = h->dmalloc((size_t)(std::max<int64_t>(1, std::max(h->n_rows, h->n_cols)) * k * es));
+    h->d_tk = h->dmalloc((size_t)(std::max<int64_t>(1, h->sum_rank) * k * es));
+  } catch (const OomError &) {
+    for (DevPhase *dp : made) {
+      cudaFree(dp->ranges);
+      dp->ranges = nullptr;
+    }
+    cudaFree(h->d_xk);
+    h->d_xk = nullptr;
+  }
+}
+
+// Whether a product of several columns can run in the multi-column kernels:
+// their scratch is there, no unit runs CTA-cooperatively (narrow_coop), and
+// neither per-launch timing nor the withheld-chunk test hook is asked for
+// (both belong to the matvec's launches).
+bool multi_ready(const bw_hmat *h, int o, int prec) {
+  if (prec > 1 || !h->d_xk || !h->d_tk || h->timing || h->withhold >= 0) return false;
+  if (h->dev[o][prec][1].n_chunks == 0 || !h->dev[o][prec][1].ranges) return false;
+  for (const DevPhase &dp : h->dev[o][prec])
+    if (dp.split.coop > dp.split.wide) return false;
+  return true;
+}
+
+// Y[:, 0:nrhs] = op X[:, 0:nrhs], nrhs <= K, in one pass over the block data:
+// x interleaved (+ permutation), phase 1, phase 2, each phase in the kernels
+// of the matvec's split.
+template <typename S, int K>
+void launch_multi(bw_hmat *h, int o, int prec, const double *X, int64_t ldx, double *Y, int64_t ldy, int nrhs,
+                  bool permuted, cudaStream_t st) {
+  using G = typename bw::Store<S>::G;
+  using L = bw::MultiLayout<S, K>;
+  static bool attr_done[64] = {};
+  smem_attr_once(attr_done, bw::stream_multi_kernel<S, K>, L::kTotal);
+  const int32_t *perm_in = permuted ? nullptr : (o == 0 ? h->d_perm1 : h->d_perm0);
+  const int32_t *perm_out = permuted ? nullptr : (o == 0 ? h->d_perm0 : h->d_perm1);
+  const int n_in = (int)h->op[o].n_in;
+  bw::gather_xk_kernel<G, K><<<(n_in + 255) / 256, 256, 0, st>>>(X, ldx, nrhs, static_cast<G *>(h->d_xk), perm_in,
+                                                                  h->dof, n_in);
+  BW_CUDA(cudaGetLastError());
+  for (int phase = 0; phase < 2; phase++) {
+    const DevPhase &dp = h->dev[o][prec][phase];
+    if (dp.n_chunks == 0) continue;
+    bw::MultiArgs m{};
+    m.s.data = dp.data;
+    m.s.chunks = dp.chunks;
+    m.s.item_ptr = dp.items;
+    m.s.queue = dp.queue;
+    m.s.y_out = Y;
+    m.s.perm_out = perm_out;
+    m.s.dof = h->dof;
+    m.s.phase = phase + 1;
+    m.s.err = h->d_err;
+    m.s.spin_limit = h->spin_limit;
+    m.xk = h->d_xk;
+    m.tk = h->d_tk;
+    m.runs = dp.gsegs;
+    m.ranges = dp.ranges;
+    m.ldy = ldy;
+    m.nrhs = nrhs;
+    if (dp.split.wide > 0) {
+      m.s.n_items = (int)dp.split.wide;
+      bw::stream_multi_kernel<S, K><<<h->grid, bw::threads_of<S>(), L::kTotal, st>>>(m);
+      BW_CUDA(cudaGetLastError());
+    }
+    if (dp.split.wide < dp.n_items) {
+      m.s.item_ptr = dp.items + dp.split.wide;
+      m.s.n_items = (int)(dp.n_items - dp.split.wide);
+      m.s.queue = dp.queue + 2;
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(2 * h->grid);
+      cfg.blockDim = dim3(32 * bw::kMultiNarrowWarps);
+      cfg.stream = st;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[0].val.programmaticStreamSerializationAllowed = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = dp.split.wide > 0 ? 1 : 0;
+      BW_CUDA(cudaLaunchKernelEx(&cfg, bw::narrow_multi_kernel<S, K>, m));
+    }
+  }
+}
+
 // One matvec with its scratch vectors in the static array (no timing).
 template <typename S>
 void launch_matvec_on(bw_hmat *h, int o, int prec, const double *x, double *y, bool permuted, cudaStream_t st,
@@ -1115,6 +1226,7 @@ int bw_finalize(bw_hmat *h, int flags) {
     if (want_mm)
       for (int o = 0; o < (want_t ? 2 : 1); o++)
         for (int ph = 0; ph < 2; ph++) upload_mm_phase(h, o, ph);
+    if (!h->plan_only) alloc_multi(h, mask, want_t);
     h->has_mm = want_mm;
     h->stored = mask;
     h->has_t = want_t;
@@ -1308,6 +1420,41 @@ int bw_matmat(bw_hmat *h, const double *X, int64_t ldx, double *Y, int64_t ldy, 
       }
       BW_CUDA(cudaSetDevice(h->device));
       launch_matmat_tc(h, o, X, ldx, Y, ldy, nrhs, (flags & BW_PERMUTED) != 0, static_cast<cudaStream_t>(stream));
+      return BW_OK;
+    });
+  }
+  const int p = prec_index(flags);
+  const char *xb = reinterpret_cast<const char *>(X), *yb = reinterpret_cast<const char *>(Y);
+  const int64_t xe = ((int64_t)(nrhs - 1) * ldx + nin) * 8, ye = ((int64_t)(nrhs - 1) * ldy + nout) * 8;
+  if (nrhs > 1 && h->finalized && !h->plan_only && p >= 0 && (h->stored & (1 << p)) && (!tr || h->has_t) &&
+      nin > 0 && nout > 0 && X && Y && (xb >= yb + ye || yb >= xb + xe) && multi_ready(h, o, p)) {
+    // passes of 8 columns; up to 4 left over go as 4, a single one as a
+    // matvec.  Columns whose X and Y ranges interleave go one by one below.
+    return guarded(h, [&] {
+      BW_CUDA(cudaSetDevice(h->device));
+      cudaStream_t st = static_cast<cudaStream_t>(stream);
+      const bool perm = (flags & BW_PERMUTED) != 0;
+      for (int c0 = 0; c0 < nrhs; c0 += bw::kMultiMax) {
+        const int nr = std::min(bw::kMultiMax, nrhs - c0);
+        const double *x = X + (int64_t)c0 * ldx;
+        double *y = Y + (int64_t)c0 * ldy;
+        if (nr == 1) {
+          if (p == 0)
+            launch_matvec<double>(h, o, 0, x, y, perm, st);
+          else
+            launch_matvec<float>(h, o, 1, x, y, perm, st);
+        } else if (nr <= 4) {
+          if (p == 0)
+            launch_multi<double, 4>(h, o, 0, x, ldx, y, ldy, nr, perm, st);
+          else
+            launch_multi<float, 4>(h, o, 1, x, ldx, y, ldy, nr, perm, st);
+        } else {
+          if (p == 0)
+            launch_multi<double, 8>(h, o, 0, x, ldx, y, ldy, nr, perm, st);
+          else
+            launch_multi<float, 8>(h, o, 1, x, ldx, y, ldy, nr, perm, st);
+        }
+      }
       return BW_OK;
     });
   }

@@ -385,7 +385,8 @@ void chunk_item(const OperatorPlan &op, const Item &it, int prec, int phase, int
   if (tiled)
     cap = std::max<int64_t>(8, std::min<int64_t>(kMaxCols, (chunk_bytes / (8 * int64_t(it.hpad) * es)) * 8));
   else
-    cap = std::max<int64_t>(1, std::min<int64_t>(kMaxCols, chunk_bytes / (int64_t(it.hpad) * es)));
+    cap = std::max<int64_t>(1, std::min<int64_t>(prec == 0 ? kMaxColsFp64 : kMaxCols,
+                                                 chunk_bytes / (int64_t(it.hpad) * es)));
   std::vector<int64_t> seg_start(it.segs.size() + 1, 0);
   for (size_t s = 0; s < it.segs.size(); s++) seg_start[s + 1] = seg_start[s] + it.segs[s].ncols;
   int64_t c0 = 0;
@@ -476,6 +477,23 @@ void build_chunks(const Problem &p, bool tr, int prec, int grid, OperatorPlan &o
       }
     }
   }
+}
+
+std::vector<std::pair<int32_t, int32_t>> run_ranges(const ChunkPlan &cp) {
+  // the runs are made chunk by chunk, so their places in G2 increase
+  std::vector<std::pair<int32_t, int32_t>> out;
+  out.reserve(cp.chunks.size());
+  for (const Chunk &c : cp.chunks) {
+    auto it = std::lower_bound(cp.gsegs.begin(), cp.gsegs.end(), c.g_off,
+                               [](const GatherSeg &g, int32_t at) { return g.dst < at; });
+    const int64_t first = it - cp.gsegs.begin();
+    int64_t count = 0, cols = 0;
+    for (; cols < c.ncols && it != cp.gsegs.end() && it->dst == c.g_off + cols; ++it, count++)
+      cols += it->cols_src & 0x7fffffffu;
+    if (cols != c.ncols) fail("the runs of a chunk do not tile its vector values");
+    out.emplace_back(i32(first, "run"), i32(count, "run count"));
+  }
+  return out;
 }
 
 namespace {

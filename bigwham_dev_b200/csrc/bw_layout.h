@@ -26,12 +26,15 @@
 
 #include <cstdint>
 #include <string>
+#include <utility>
 #include <vector>
 
 namespace bw {
 
 constexpr int kStageBytes = 32768;   // bytes of block data per pipeline stage
 constexpr int kMaxCols = 512;        // columns per chunk (size of a stage's gather buffer)
+constexpr int kMaxColsFp64 = 256;    // FP64 chunks (items of 8 rows would reach 512): 8 columns of a
+                                     // right-hand-side window then fit a 16 KB stage, as in FP32
 constexpr int kHMax = 512;           // max padded rows of one item
 constexpr int kRowAlign = 8;         // padded rows are a multiple of this
 constexpr int kItemAlign = 64;       // item start alignment, in elements
@@ -194,6 +197,11 @@ void compute_scales(const Problem &p, bool transposed, bool check_finite, Operat
 // into chunks, and orders the items longest first (cost = bytes + a per-chunk
 // overhead): the kernel's CTAs take them in that order from a device queue.
 void build_chunks(const Problem &p, bool transposed, int prec, int grid, OperatorPlan &op);
+
+// Each chunk's runs in a phase-2 plan's run list, in the chunks' order: (first
+// run, number of runs).  The runs of a chunk are consecutive and tile its slice
+// of the vector values in order (std::runtime_error otherwise).
+std::vector<std::pair<int32_t, int32_t>> run_ranges(const ChunkPlan &cp);
 
 // Writes the data of items [i_begin, i_end) of one phase, converted to the
 // precision and in its layout, into dst (dst[0] is element `base` of the
