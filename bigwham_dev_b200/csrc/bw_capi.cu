@@ -1747,7 +1747,7 @@ void par_copy(void *dst, const void *src, int64_t bytes) {
 // Shared checks and launch of the observation-field kernels.
 template <typename Launch>
 int fields_entry(const char *name, int device, int64_t n_elems, const double *records, const double *dd, double G,
-                 double nu, int64_t n_pts, const double *pts, const double *stress, const double *disp, int threads,
+                 double nu, int64_t n_pts, const double *pts, const double *stress, const double *disp,
                  Launch &&launch) {
   return device_guarded([&] {
     if (!records || !dd || n_elems < 1 || n_pts < 0 || (n_pts > 0 && (!pts || (!stress && !disp))))
@@ -1756,10 +1756,8 @@ int fields_entry(const char *name, int device, int64_t n_elems, const double *re
     if (!(G > 0.0) || !(nu > -1.0 && nu < 0.5)) throw std::invalid_argument(std::string(name) + ": bad G or nu");
     if (n_pts == 0) return BW_OK;
     BW_CUDA(cudaSetDevice(device));
-    int sms = 0;
-    BW_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    const int64_t need = (n_pts + threads - 1) / threads;
-    launch(static_cast<int>(std::min<int64_t>(need, int64_t(std::max(1, sms)) * 4)));
+    const int lanes = bw::field_lanes(n_pts), per_cta = bw::kFieldThreads / lanes;
+    launch(static_cast<int>(std::min<int64_t>((n_pts + per_cta - 1) / per_cta, int64_t(1) << 30)), lanes);
     BW_CUDA(cudaGetLastError());
     return BW_OK;
   });
@@ -1943,10 +1941,13 @@ int bw_create_from_file(const char *path, int device, int verify, bw_hmat **out)
 
 int bw_s0_fields(int device, int64_t n_elems, const double *records, const double *dd, double G, double nu,
                  int64_t n_pts, const double *pts, double *stress, double *disp, void *stream) {
-  return fields_entry("bw_s0_fields", device, n_elems, records, dd, G, nu, n_pts, pts, stress, disp, bw::kS0Threads,
-                      [&](int grid) {
-                        bw::s0_fields_kernel<<<grid, bw::kS0Threads, 0, static_cast<cudaStream_t>(stream)>>>(
-                            records, dd, static_cast<int>(n_elems), pts, static_cast<long long>(n_pts), G, nu,
+  return fields_entry("bw_s0_fields", device, n_elems, records, dd, G, nu, n_pts, pts, stress, disp,
+                      [&](int grid, int lanes) {
+                        auto *k = stress && disp ? bw::s0_fields_kernel<true, true>
+                                  : stress       ? bw::s0_fields_kernel<true, false>
+                                                 : bw::s0_fields_kernel<false, true>;
+                        k<<<grid, bw::kFieldThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+                            records, dd, static_cast<int>(n_elems), pts, static_cast<long long>(n_pts), G, nu, lanes,
                             stress, disp);
                       });
 }
@@ -1954,9 +1955,12 @@ int bw_s0_fields(int device, int64_t n_elems, const double *records, const doubl
 int bw_r0_fields(int device, int64_t n_elems, const double *records, const double *dd, double G, double nu,
                  int64_t n_pts, const double *pts, double *stress, double *disp, void *stream) {
   return fields_entry("bw_r0_fields", device, n_elems, records, dd, G, nu, n_pts, pts, stress, disp,
-                      bw::kR0FieldThreads, [&](int grid) {
-                        bw::r0_fields_kernel<<<grid, bw::kR0FieldThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-                            records, dd, static_cast<int>(n_elems), pts, static_cast<long long>(n_pts), G, nu,
+                      [&](int grid, int lanes) {
+                        auto *k = stress && disp ? bw::r0_fields_kernel<true, true>
+                                  : stress       ? bw::r0_fields_kernel<true, false>
+                                                 : bw::r0_fields_kernel<false, true>;
+                        k<<<grid, bw::kFieldThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+                            records, dd, static_cast<int>(n_elems), pts, static_cast<long long>(n_pts), G, nu, lanes,
                             stress, disp);
                       });
 }

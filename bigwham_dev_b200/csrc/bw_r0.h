@@ -71,38 +71,89 @@ constexpr double kPi = 3.14159265358979323846;
 // R + Y without cancellation (q = X^2 + z^2).
 BW_HD double r_plus(double R, double Y, double q) { return Y >= 0.0 ? R + Y : q / (R - Y); }
 
-// Off the element plane (z != 0): every derivative up to third order.
+// 1 / sqrt(v).
+BW_HD double inv_sqrt(double v) {
+#ifdef __CUDA_ARCH__
+  return rsqrt(v);
+#else
+  return 1.0 / sqrt(v);
+#endif
+}
+
+// One Newton step of a reciprocal: r ~ 1 / v to a few roundings -> 1 / v to
+// half of one more.  The corner sums cancel, so the few ulp that a shared
+// division leaves in its factors would show in the stresses.
+BW_HD double refine_inv(double v, double r) { return fma(r, fma(-v, r, 1.0), r); }
+
+// Off the element plane (z != 0): every derivative up to third order.  The
+// logarithms of the corners combine into one of their ratio per direction, the
+// arctangents into one per side (each sum of two lies within +-pi, so atan2 of
+// the complex product gives it without a branch), and the divisions into six:
+// one for the two X^2 + z^2, one for the two Y^2 + z^2 and one per corner for
+// 1 / (R + |X|) and 1 / (R + |Y|) together (some 80 with every term by itself).  With P = R (R + Y), p = 1 / P and
+// k = 2 + Y / R:
+//   F_xx = X p, F_xz = z p, F_xxx = (P - X^2 k) p^2, F_xzz = (P - z^2 k) p^2,
+//   F_xxz = -X z k p^2.
 BW_HD Derivs derivs_offplane(double x, double y, double z, double a, double b) {
   Derivs d = {};
+  const double Xc[2] = {x + a, x - a}, Yc[2] = {y + b, y - b};
+  const double z2 = z * z;
+  const double qx[2] = {Xc[0] * Xc[0] + z2, Xc[1] * Xc[1] + z2}, qy[2] = {Yc[0] * Yc[0] + z2, Yc[1] * Yc[1] + z2};
+  // one division per pair (for all four together the product would leave the
+  // range that the R^4 below needs anyway)
+  const double ivx = 1.0 / (qx[0] * qx[1]), ivy = 1.0 / (qy[0] * qy[1]);
+  const double iqx[2] = {refine_inv(qx[0], ivx * qx[1]), refine_inv(qx[1], ivx * qx[0])};
+  const double iqy[2] = {refine_inv(qy[0], ivy * qy[1]), refine_inv(qy[1], ivy * qy[0])};
+  double lx = 1.0, ly = 1.0;  // ratios under the logarithms
   for (int cx = 0; cx < 2; cx++) {
+    double re = 1.0, im = 0.0;  // product of the side's corners, angle = sum of its arctangents
     for (int cy = 0; cy < 2; cy++) {
-      const double sx = cx ? -1.0 : 1.0, sy = cy ? -1.0 : 1.0, s = sx * sy;
-      const double X = x + sx * a, Y = y + sy * b;
-      const double X2 = X * X, Y2 = Y * Y, z2 = z * z;
-      const double R = sqrt(X2 + Y2 + z2), R2 = R * R, R3 = R2 * R;
-      const double qx = X2 + z2, qy = Y2 + z2;
-      const double RY = r_plus(R, Y, qx), RX = r_plus(R, X, qy);
-      d.x += s * log(RY);
-      d.y += s * log(RX);
-      d.z -= s * atan(X * Y / (z * R));
-      d.xx += s * X / (R * RY);
-      d.yy += s * Y / (R * RX);
-      d.xy += s / R;
-      d.xz += s * z / (R * RY);
-      d.yz += s * z / (R * RX);
-      d.zz += s * X * Y * (X2 + Y2 + 2.0 * z2) / (R * qx * qy);
-      d.xxy -= s * X / R3;
-      d.xyy -= s * Y / R3;
-      d.xyz -= s * z / R3;
-      const double RY2 = RY * RY, RX2 = RX * RX;
-      d.xxx += s * (R * RY - X2 * (2.0 * R + Y) / R) / (R2 * RY2);
-      d.yyy += s * (R * RX - Y2 * (2.0 * R + X) / R) / (R2 * RX2);
-      d.xxz -= s * X * z * (2.0 * R + Y) / (R3 * RY2);
-      d.yyz -= s * Y * z * (2.0 * R + X) / (R3 * RX2);
-      d.xzz += s * (R * RY - z2 * (2.0 * R + Y) / R) / (R2 * RY2);
-      d.yzz += s * (R * RX - z2 * (2.0 * R + X) / R) / (R2 * RX2);
+      const double s = (cx == cy) ? 1.0 : -1.0;
+      const double X = Xc[cx], Y = Yc[cy], R2 = X * X + qy[cy];
+      const double i0 = inv_sqrt(R2), r0 = R2 * i0;
+      const double R = fma(0.5 * i0, fma(-r0, r0, R2), r0);  // sqrt(R2)
+      const double iR = refine_inv(R, i0);
+      const double sX = R + fabs(X), sY = R + fabs(Y);  // no cancellation
+      const double h = 1.0 / (sX * sY);
+      // R + Y and its reciprocal (for Y < 0: (X^2 + z^2) / (R - Y)); likewise R + X
+      const double iX = refine_inv(sX, sY * h), iY = refine_inv(sY, sX * h);
+      const double RY = Y >= 0.0 ? sY : qx[cx] * iY, iRY = Y >= 0.0 ? iY : sY * iqx[cx];
+      const double RX = X >= 0.0 ? sX : qy[cy] * iX, iRX = X >= 0.0 ? iX : sX * iqy[cy];
+      lx *= cx == cy ? RY : iRY;
+      ly *= cx == cy ? RX : iRX;
+      const double ar = fabs(z) * R, ai = cx == cy ? X * Y : -(X * Y);
+      const double nr = re * ar - im * ai;
+      im = re * ai + im * ar;
+      re = nr;
+      const double iR3 = iR * iR * iR, P = R * RY, Q = R * RX;
+      const double p = refine_inv(P, iR * iRY), q = refine_inv(Q, iR * iRX);
+      const double p2 = p * p, q2 = q * q, kp = 2.0 + Y * iR, kq = 2.0 + X * iR;
+      d.xx += s * (X * p);
+      d.yy += s * (Y * q);
+      d.xy += s * iR;
+      d.xz += s * p;   // times z below, as the other terms odd in z
+      d.yz += s * q;
+      d.zz += s * (X * Y * (qx[cx] + qy[cy]) * iR * (iqx[cx] * iqy[cy]));
+      d.xxy -= s * (X * iR3);
+      d.xyy -= s * (Y * iR3);
+      d.xyz -= s * iR3;
+      d.xxx += s * ((P - X * X * kp) * p2);
+      d.yyy += s * ((Q - Y * Y * kq) * q2);
+      d.xxz -= s * (X * kp * p2);
+      d.yyz -= s * (Y * kq * q2);
+      d.xzz += s * ((P - z2 * kp) * p2);
+      d.yzz += s * ((Q - z2 * kq) * q2);
     }
+    d.z -= atan2(im, re);
   }
+  d.x = log(lx);
+  d.y = log(ly);
+  if (z < 0.0) d.z = -d.z;
+  d.xz *= z;
+  d.yz *= z;
+  d.xyz *= z;
+  d.xxz *= z;
+  d.yyz *= z;
   d.zzz = -(d.xxz + d.yyz);
   return d;
 }

@@ -20,7 +20,10 @@ namespace r0 {
 // row-major (9), half sides a, b; then the local DD (3).
 constexpr int kFieldDoubles = 17;
 
-// el: kFieldDoubles values as above; acc += the 9 field values at p.
+// el: kFieldDoubles values as above; acc += the 9 field values at p.  The DD
+// contracts with the derivatives directly (bw_r0.h's table of stresses and
+// displacements, with the coefficients of each derivative collected).
+template <bool kStress = true, bool kDisp = true>
 BW_HD void add_point_fields(const double *el, const double *p, double G, double nu, double acc[9]) {
   const double *cp = el, *R = el + 3, *dd = el + 14;
   const double a = el[12], b = el[13];
@@ -28,25 +31,41 @@ BW_HD void add_point_fields(const double *el, const double *p, double G, double 
   for (int k = 0; k < 3; k++) d[k] = p[k] - cp[k];
   for (int i = 0; i < 3; i++) l[i] = R[3 * i] * d[0] + R[3 * i + 1] * d[1] + R[3 * i + 2] * d[2];
   const Derivs D = derivs(l[0], l[1], l[2], a, b);
-  double s[3][6], u[3][3];
-  stress_from(D, l[2], G, nu, s);
-  displacement_from(D, l[2], nu, u);
-  double c[6];  // local stress: xx, yy, zz, xy, xz, yz
-  for (int q = 0; q < 6; q++) c[q] = s[0][q] * dd[0] + s[1][q] * dd[1] + s[2][q] * dd[2];
-  const double S[3][3] = {{c[0], c[3], c[4]}, {c[3], c[1], c[5]}, {c[4], c[5], c[2]}};
-  double T[3][3];  // S R
-  for (int i = 0; i < 3; i++)
-    for (int j = 0; j < 3; j++) T[i][j] = S[i][0] * R[j] + S[i][1] * R[3 + j] + S[i][2] * R[6 + j];
-  auto g = [&](int i, int j) { return R[i] * T[0][j] + R[3 + i] * T[1][j] + R[6 + i] * T[2][j]; };  // (R^T S R)_ij
-  acc[0] += g(0, 0);
-  acc[1] += g(1, 1);
-  acc[2] += g(2, 2);
-  acc[3] += g(0, 1);
-  acc[4] += g(0, 2);
-  acc[5] += g(1, 2);
-  double ul[3];
-  for (int i = 0; i < 3; i++) ul[i] = u[i][0] * dd[0] + u[i][1] * dd[1] + u[i][2] * dd[2];
-  for (int i = 0; i < 3; i++) acc[6 + i] += R[i] * ul[0] + R[3 + i] * ul[1] + R[6 + i] * ul[2];
+  const double z = l[2], k2 = 1.0 - 2.0 * nu;
+  if (kStress) {
+    const double C = G / (4.0 * kPi * (1.0 - nu));
+    const double dx = C * dd[0], dy = C * dd[1], dz = C * dd[2];
+    const double zx = z * dx, zy = z * dy, zd = z * dz;
+    const double sxx = 2.0 * dx * D.xz + 2.0 * nu * dy * D.yz + dz * (D.zz + k2 * D.yy) -
+                       (zx * D.xxx + zy * D.xxy + zd * D.xxz);
+    const double syy = 2.0 * nu * dx * D.xz + 2.0 * dy * D.yz + dz * (D.zz + k2 * D.xx) -
+                       (zx * D.xyy + zy * D.yyy + zd * D.yyz);
+    const double szz = dz * D.zz - (zx * D.xzz + zy * D.yzz + zd * D.zzz);
+    const double sxy = (1.0 - nu) * (dx * D.yz + dy * D.xz) - k2 * dz * D.xy -
+                       (zx * D.xxy + zy * D.xyy + zd * D.xyz);
+    const double sxz = dx * (D.zz + nu * D.yy) - nu * dy * D.xy - (zx * D.xxz + zy * D.xyz + zd * D.xzz);
+    const double syz = dy * (D.zz + nu * D.xx) - nu * dx * D.xy - (zx * D.xyz + zy * D.yyz + zd * D.yzz);
+    const double S[3][3] = {{sxx, sxy, sxz}, {sxy, syy, syz}, {sxz, syz, szz}};
+    double T[3][3];  // S R
+    for (int i = 0; i < 3; i++)
+      for (int j = 0; j < 3; j++) T[i][j] = S[i][0] * R[j] + S[i][1] * R[3 + j] + S[i][2] * R[6 + j];
+    auto g = [&](int i, int j) { return R[i] * T[0][j] + R[3 + i] * T[1][j] + R[6 + i] * T[2][j]; };  // (R^T S R)_ij
+    acc[0] += g(0, 0);
+    acc[1] += g(1, 1);
+    acc[2] += g(2, 2);
+    acc[3] += g(0, 1);
+    acc[4] += g(0, 2);
+    acc[5] += g(1, 2);
+  }
+  if (kDisp) {
+    const double c = 1.0 / (8.0 * kPi * (1.0 - nu)), k1 = 2.0 * (1.0 - nu);
+    const double ux = c * dd[0], uy = c * dd[1], uz = c * dd[2];
+    const double ul[3] = {
+        ux * (k1 * D.z - z * D.xx) - uy * (z * D.xy) - uz * (k2 * D.x + z * D.xz),
+        uy * (k1 * D.z - z * D.yy) - ux * (z * D.xy) - uz * (k2 * D.y + z * D.yz),
+        ux * (k2 * D.x - z * D.xz) + uy * (k2 * D.y - z * D.yz) + uz * (k1 * D.z - z * D.zz)};
+    for (int i = 0; i < 3; i++) acc[6 + i] += R[i] * ul[0] + R[3 + i] * ul[1] + R[6 + i] * ul[2];
+  }
 }
 
 }  // namespace r0

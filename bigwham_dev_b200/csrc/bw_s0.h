@@ -41,64 +41,86 @@ namespace s0 {
 constexpr int kRecordDoubles = 5;  // cx, cy, a, tx, ty
 constexpr double kPi = 3.14159265358979323846;
 
+// Derivatives of F = f / c (f_xx = -f_yy).  With z = x + i y, both end points
+// combine into one complex reciprocal,
+//   1 / (z - a) - 1 / (z + a) = 2 a / zeta,          zeta = z^2 - a^2,
+//   1 / (z - a)^2 - 1 / (z + a)^2 = 4 a z / zeta^2,
+// |zeta|^2 = r1^2 r2^2, whose parts are the second and third derivatives; the
+// two logarithms are one of the ratio and the two angles one, the angle the
+// segment subtends.  A pair costs one division, one log and one atan2 (eight
+// divisions and two of each when every term is taken by itself), and the far
+// field loses no digits to the difference of two nearly equal ends.
 struct Derivs {
-  double fx, fy, fxy, fyy, fxyy, fyyy;  // f_xx = -f_yy
+  double fx, fy, fxy, fyy, fxyy, fyyy;
 };
 
-BW_S0_HD Derivs derivs(double x, double y, double a, double nu) {
-  const double c = 1.0 / (4.0 * kPi * (1.0 - nu));
+BW_S0_HD Derivs derivs(double x, double y, double a) {
   const double xm = x - a, xp = x + a, y2 = y * y;
-  const double r1 = xm * xm + y2, r2 = xp * xp + y2;
-  const double ys = (y == 0.0) ? -0.0 : y;  // on the line: the limit from below
+  const double r1 = xm * xm + y2, r2 = xp * xp + y2;  // squared distances to the ends
+  const double w = 1.0 / (r1 * r2);
+  const double zr = xm * xp - y2, zi = 2.0 * x * y;   // zeta, no cancellation near an end
+  const double gr = zr * w, gi = -zi * w;             // 1 / zeta
+  const double hr = gr * gr - gi * gi, hi = 2.0 * gr * gi;
+  const double ys = (y == 0.0) ? -0.0 : y;            // on the line: the limit from below
   Derivs d;
-  d.fx = 0.5 * c * (log(r1) - log(r2));
-  d.fy = -c * (atan2(ys, xm) - atan2(ys, xp));
-  d.fxy = c * (y / r1 - y / r2);
-  d.fyy = -c * (xm / r1 - xp / r2);
-  d.fxyy = c * ((xm * xm - y2) / (r1 * r1) - (xp * xp - y2) / (r2 * r2));
-  d.fyyy = 2.0 * c * y * (xm / (r1 * r1) - xp / (r2 * r2));
+  d.fx = 0.5 * log(r1 * r1 * w);
+  d.fy = -atan2(2.0 * a * ys, xm * xp + y2);
+  d.fyy = -2.0 * a * gr;
+  d.fxy = -2.0 * a * gi;
+  d.fxyy = 4.0 * a * (x * hr - y * hi);
+  d.fyyy = -4.0 * a * (x * hi + y * hr);
   return d;
 }
 
-// Local fields of unit DDs: s[k] = (sxx, syy, sxy), u[k] = (ux, uy) for the DD
-// k = 0 (shear, along t) and k = 1 (normal, along n).
-BW_S0_HD void local_fields(double x, double y, double a, double G, double nu, double s[2][3], double u[2][2]) {
-  const Derivs d = derivs(x, y, a, nu);
-  const double fxx = -d.fyy;
-  s[0][0] = 2.0 * G * (2.0 * d.fxy + y * d.fxyy);
-  s[0][1] = 2.0 * G * (-y * d.fxyy);
-  s[0][2] = 2.0 * G * (d.fyy + y * d.fyyy);
-  s[1][0] = 2.0 * G * (d.fyy + y * d.fyyy);
-  s[1][1] = 2.0 * G * (d.fyy - y * d.fyyy);
-  s[1][2] = 2.0 * G * (-y * d.fxyy);
-  u[0][0] = 2.0 * (1.0 - nu) * d.fy - y * fxx;
-  u[0][1] = (1.0 - 2.0 * nu) * d.fx - y * d.fxy;
-  u[1][0] = -(1.0 - 2.0 * nu) * d.fx - y * d.fxy;
-  u[1][1] = 2.0 * (1.0 - nu) * d.fy - y * d.fyy;
+// What a field evaluation reads of an element: centre, half length, tangent,
+// cosine and sine of its double angle, the local DD over 4 pi (1 - nu).
+constexpr int kFieldDoubles = 9;
+
+BW_S0_HD void field_data(const double *rec, double dd_s, double dd_n, double nu, double *el) {
+  const double tx = rec[3], ty = rec[4], c = 1.0 / (4.0 * kPi * (1.0 - nu));
+  for (int k = 0; k < 5; k++) el[k] = rec[k];
+  el[5] = tx * tx - ty * ty;
+  el[6] = 2.0 * tx * ty;
+  el[7] = c * dd_s;
+  el[8] = c * dd_n;
 }
 
 // Global stress (s11, s22, s12) and displacement (u1, u2) at point (px, py)
-// due to the element `rec` carrying the local DD (dd_s, dd_n); added to acc
-// (5 values: s11, s22, s12, u1, u2).
+// due to the element `el` (field_data), added to acc (5 values: s11, s22, s12,
+// u1, u2).  The local stress enters through its mean m, half difference h and
+// shear q, which rotate by the double angle.
+template <bool kStress, bool kDisp>
+BW_S0_HD void add_fields(const double *el, double px, double py, double G, double nu, double acc[5]) {
+  const double tx = el[3], ty = el[4], us = el[7], un = el[8];
+  const double dx = px - el[0], dy = py - el[1];
+  const double x = tx * dx + ty * dy, y = tx * dy - ty * dx;
+  const Derivs d = derivs(x, y, el[2]);
+  if (kStress) {
+    const double ks = 2.0 * G * us, kn = 2.0 * G * un;
+    const double p = y * d.fxyy, r = y * d.fyyy;
+    // sxx = ks (2 fxy + p) + kn (fyy + r), syy = -ks p + kn (fyy - r), sxy = ks (fyy + r) - kn p
+    const double m = ks * d.fxy + kn * d.fyy, h = ks * (d.fxy + p) + kn * r, q = ks * (d.fyy + r) - kn * p;
+    const double v = h * el[5] - q * el[6];
+    acc[0] += m + v;
+    acc[1] += m - v;
+    acc[2] += h * el[6] + q * el[5];
+  }
+  if (kDisp) {
+    const double k1 = 2.0 * (1.0 - nu), k2 = 1.0 - 2.0 * nu;
+    const double ux = us * (k1 * d.fy + y * d.fyy) - un * (k2 * d.fx + y * d.fxy);
+    const double uy = us * (k2 * d.fx - y * d.fxy) + un * (k1 * d.fy - y * d.fyy);
+    acc[3] += ux * tx - uy * ty;
+    acc[4] += ux * ty + uy * tx;
+  }
+}
+
+// The same from the element's record and its local DD (dd_s, dd_n).
+template <bool kStress = true, bool kDisp = true>
 BW_S0_HD void add_point_fields(const double *rec, double dd_s, double dd_n, double px, double py, double G,
                                double nu, double acc[5]) {
-  const double cx = rec[0], cy = rec[1], a = rec[2], tx = rec[3], ty = rec[4];
-  const double nx = -ty, ny = tx;
-  const double dx = px - cx, dy = py - cy;
-  const double xl = tx * dx + ty * dy, yl = nx * dx + ny * dy;
-  double s[2][3], u[2][2];
-  local_fields(xl, yl, a, G, nu, s, u);
-  const double sxx = s[0][0] * dd_s + s[1][0] * dd_n;
-  const double syy = s[0][1] * dd_s + s[1][1] * dd_n;
-  const double sxy = s[0][2] * dd_s + s[1][2] * dd_n;
-  const double ux = u[0][0] * dd_s + u[1][0] * dd_n;
-  const double uy = u[0][1] * dd_s + u[1][1] * dd_n;
-  // R^T S R = sxx t t^T + syy n n^T + sxy (t n^T + n t^T); R^T u = ux t + uy n
-  acc[0] += sxx * tx * tx + syy * nx * nx + 2.0 * sxy * tx * nx;
-  acc[1] += sxx * ty * ty + syy * ny * ny + 2.0 * sxy * ty * ny;
-  acc[2] += sxx * tx * ty + syy * nx * ny + sxy * (tx * ny + nx * ty);
-  acc[3] += ux * tx + uy * nx;
-  acc[4] += ux * ty + uy * ny;
+  double el[kFieldDoubles];
+  field_data(rec, dd_s, dd_n, nu, el);
+  add_fields<kStress, kDisp>(el, px, py, G, nu, acc);
 }
 
 // Hypersingular (H) entry between two elements: tractions at the receiver's
@@ -111,7 +133,7 @@ BW_S0_HD void h_entry(const double *src, const double *rcv, double G, double nu,
   const double tx = rcv[3], ty = rcv[4], nx = -ty, ny = tx;
   for (int k = 0; k < 2; k++) {
     double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    add_point_fields(src, k == 0 ? 1.0 : 0.0, k == 1 ? 1.0 : 0.0, rcv[0], rcv[1], G, nu, acc);
+    add_point_fields<true, false>(src, k == 0 ? 1.0 : 0.0, k == 1 ? 1.0 : 0.0, rcv[0], rcv[1], G, nu, acc);
     const double t1 = acc[0] * nx + acc[2] * ny, t2 = acc[2] * nx + acc[1] * ny;  // sigma n
     K[0][k] = t1 * tx + t2 * ty;
     K[1][k] = t1 * nx + t2 * ny;
