@@ -1,16 +1,26 @@
 // Device block ACA of the admissible blocks of a 3DR0-H H-matrix.
 //
-// One CTA compresses one block at a time (grid-stride over blocks), running
-// the steps of bw::aca::block_aca_host with the work of each step spread over
-// the CTA's threads:
+// One CTA compresses one block at a time, running the steps of
+// bw::aca::block_aca_host with the work of each step spread over the CTA's
+// threads:
 //   * residual row / column bands: one thread per point pair (kernel entry +
 //     the subtraction of the current approximation);
 //   * pivot searches: per-thread smallest singular values, then a CTA argmax
 //     that keeps the first index on ties (the reference scans in order and
 //     replaces only on a strictly larger value);
-//   * Frobenius terms: CTA reductions of 3 x 3 Gram blocks.
-// Every stop decision is taken by thread 0 and broadcast through shared
-// memory, so all threads leave the loop together.  Factor storage per block is
+//   * Frobenius terms of the new rank block with every earlier one and with
+//     itself, together: A_r^T A_k by a warp per r, lanes along A's contiguous
+//     columns; B_k B_r^T by a lane per r, which B's storage keeps side by
+//     side, warps along the points.
+// The arithmetic is small (about 1 GFLOP for a 64 x 64 crack); a step's time is
+// the latency of what it does one after the other, so the steps have a fixed
+// number of barriers (ten, at any rank: two CTA reductions per earlier rank
+// block took most of the time before), and the blocks come from a queue,
+// longest first, so that the largest does not start last.
+// A 64 x 64 crack's 1,584 blocks with the full-rank blocks: 28.0 -> 19.4 ms
+// through DeviceKernels.
+// Every stop decision is taken from values in shared memory that all threads
+// read, so all threads leave the loop together.  Factor storage per block is
 // capacity-bounded (cap blocks of rank); a block that needs more reports
 // rank -1 and writes nothing past its capacity.
 #pragma once
@@ -21,6 +31,7 @@
 namespace bw {
 
 constexpr int kAcaThreads = 128;
+constexpr int kAcaWarps = kAcaThreads / 32;
 
 struct AcaBlock {
   long long a_off, b_off;  // factor storage (doubles): A n0 3 x cap 3, B cap 3 x n1 3, column-major
@@ -31,39 +42,134 @@ struct AcaBlock {
 
 // CTA argmax of (value, index) pairs: largest value, smallest index on ties;
 // index -1 when no thread had a candidate.
-__device__ __forceinline__ void aca_argmax(double v, int idx, double *sv, int *si, double &best, int &bi) {
-  const int t = threadIdx.x;
-  sv[t] = v;
-  si[t] = idx;
-  __syncthreads();
-  for (int s = kAcaThreads / 2; s > 0; s >>= 1) {
-    if (t < s) {
-      const double v2 = sv[t + s];
-      const int i2 = si[t + s];
-      if (i2 >= 0 && (si[t] < 0 || v2 > sv[t] || (v2 == sv[t] && i2 < si[t]))) {
-        sv[t] = v2;
-        si[t] = i2;
-      }
+__device__ __forceinline__ void aca_argmax(double v, int idx, double *sv, int *si, int &bi) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  auto better = [](double v2, int i2, double v1, int i1) {
+    return i2 >= 0 && (i1 < 0 || v2 > v1 || (v2 == v1 && i2 < i1));
+  };
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double v2 = __shfl_xor_sync(0xffffffffu, v, o);
+    const int i2 = __shfl_xor_sync(0xffffffffu, idx, o);
+    if (better(v2, i2, v, idx)) {
+      v = v2;
+      idx = i2;
     }
-    __syncthreads();
   }
-  best = sv[0];
+  if (lane == 0) {
+    sv[warp] = v;
+    si[warp] = idx;
+  }
+  __syncthreads();
   bi = si[0];
+  double best = sv[0];
+  for (int w = 1; w < kAcaWarps; w++)
+    if (better(sv[w], si[w], best, bi)) {
+      best = sv[w];
+      bi = si[w];
+    }
   __syncthreads();
 }
 
-// CTA sum of 9 partial values per thread into out[9] (all threads see it).
-__device__ __forceinline__ void aca_sum9(const double *part, double *red, double *out) {
-  const int t = threadIdx.x;
-  for (int k = 0; k < 9; k++) red[k * kAcaThreads + t] = part[k];
-  __syncthreads();
-  for (int s = kAcaThreads / 2; s > 0; s >>= 1) {
-    if (t < s)
-      for (int k = 0; k < 9; k++) red[k * kAcaThreads + t] += red[k * kAcaThreads + t + s];
-    __syncthreads();
+// K -= A B over `rank` scalar columns: A's three rows of one point, B's three
+// columns of another.
+__device__ __forceinline__ void aca_subtract(const double *A, long long lda, const double *B, long long ldb, int rank,
+                                             double (&K)[3][3]) {
+#pragma unroll 3
+  for (int k = 0; k < rank; k++) {
+    const double a0 = A[k * lda], a1 = A[k * lda + 1], a2 = A[k * lda + 2];
+#pragma unroll
+    for (int b = 0; b < 3; b++) {
+      const double v = B[b * ldb + k];
+      K[0][b] -= a0 * v;
+      K[1][b] -= a1 * v;
+      K[2][b] -= a2 * v;
+    }
   }
-  for (int k = 0; k < 9; k++) out[k] = red[k * kAcaThreads];
-  __syncthreads();
+}
+
+constexpr int kAcaPass = 32;  // earlier rank blocks whose Frobenius terms one pass takes (a lane each)
+
+struct AcaFrob {
+  double m1[kAcaPass][9];             // A_r^T A_k
+  double m2[kAcaWarps][9][kAcaPass];  // per warp: part of (B_k B_r^T)^T
+};
+
+// Frobenius products <A_r B_r, A_k B_k>_F for r = 0 .. k: their sum over r < k
+// in `cross` and the term r = k in `self` (all threads).
+__device__ __forceinline__ void aca_frobenius(const double *A, long long lda, const double *B, long long ldb, int k,
+                                              long long cols, AcaFrob &f, double *s_out, double &cross,
+                                              double &self) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  cross = 0.0;
+  self = 0.0;
+  const double *Ak = A + 3LL * k * lda;
+  for (int r0 = 0; r0 <= k; r0 += kAcaPass) {
+    const int nr = min(kAcaPass, k + 1 - r0);
+    // warp: one r at a time, lanes along the rows
+    for (int q = warp; q < nr; q += kAcaWarps) {
+      const double *Ar = A + 3LL * (r0 + q) * lda;
+      double m[9] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+      for (long long i = lane; i < lda; i += 32) {
+        const double a0 = Ar[i], a1 = Ar[lda + i], a2 = Ar[2 * lda + i];
+#pragma unroll
+        for (int b = 0; b < 3; b++) {
+          const double v = Ak[b * lda + i];
+          m[3 * b] += a0 * v;
+          m[3 * b + 1] += a1 * v;
+          m[3 * b + 2] += a2 * v;
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < 9; e++)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m[e] += __shfl_xor_sync(0xffffffffu, m[e], o);
+      if (lane == 0)
+#pragma unroll
+        for (int e = 0; e < 9; e++) f.m1[q][e] = m[e];
+    }
+    // lane: one r, warps along the columns
+    double m[9] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    if (lane < nr) {
+      const double *Br = B + 3LL * (r0 + lane), *Bk = B + 3LL * k;
+#pragma unroll 2
+      for (long long j = warp; j < cols; j += kAcaWarps) {
+        const double *c = Br + j * ldb, *d = Bk + j * ldb;
+        const double a0 = c[0], a1 = c[1], a2 = c[2];
+#pragma unroll
+        for (int b = 0; b < 3; b++) {
+          m[3 * b] += a0 * d[b];
+          m[3 * b + 1] += a1 * d[b];
+          m[3 * b + 2] += a2 * d[b];
+        }
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 9; e++) f.m2[warp][e][lane] = m[e];
+    __syncthreads();
+    if (warp == 0) {
+      double v = 0.0;
+      if (lane < nr)
+#pragma unroll
+        for (int e = 0; e < 9; e++) {
+          double m2 = f.m2[0][e][lane];
+          for (int w = 1; w < kAcaWarps; w++) m2 += f.m2[w][e][lane];
+          v += f.m1[lane][e] * m2;
+        }
+      const bool last = r0 + lane == k;
+      const double own = __shfl_sync(0xffffffffu, v, (k - r0) & 31);
+      v = last || lane >= nr ? 0.0 : v;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (lane == 0) {
+        s_out[0] = v;
+        s_out[1] = own;
+      }
+    }
+    __syncthreads();
+    cross += s_out[0];
+    self = s_out[1];  // the last pass holds r = k
+  }
 }
 
 __global__ void __launch_bounds__(kAcaThreads) r0_aca_kernel(const double *__restrict__ records,
@@ -71,16 +177,21 @@ __global__ void __launch_bounds__(kAcaThreads) r0_aca_kernel(const double *__res
                                                              const AcaBlock *__restrict__ blocks, int n_blocks,
                                                              double G, double nu, double eps, double *factors_a,
                                                              double *factors_b, double *scratch,
-                                                             long long slot_doubles, int *rank_out,
-                                                             double *err_out) {
-  __shared__ double s_val[kAcaThreads];
-  __shared__ int s_idx[kAcaThreads];
-  __shared__ double s_red[9 * kAcaThreads];
-  __shared__ double s_gamma[9];
-  __shared__ int s_ctl[4];  // [0] continue, [1] next row block, [2] pivot column block
+                                                             long long slot_doubles, const int *order, int *queue,
+                                                             int *rank_out, double *err_out) {
+  __shared__ double s_val[kAcaWarps];
+  __shared__ int s_idx[kAcaWarps];
+  __shared__ AcaFrob s_frob;
+  __shared__ double s_gamma[9], s_sum[2];
+  __shared__ int s_ctl[2];  // [0] continue, [1] the CTA's next block
   const int t = threadIdx.x;
   double *row = scratch + (long long)blockIdx.x * slot_doubles;  // 3 x n1 3 (ld 3)
-  for (int bk = blockIdx.x; bk < n_blocks; bk += gridDim.x) {
+  for (;;) {
+    if (t == 0) s_ctl[1] = atomicAdd(queue, 1);
+    __syncthreads();
+    const int place = s_ctl[1];
+    if (place >= n_blocks) break;
+    const int bk = order[place];
     const AcaBlock B_ = blocks[bk];
     const int n0 = B_.n0, n1 = B_.n1, cap = B_.cap;
     const long long lda = 3LL * n0, ldb = 3LL * cap;
@@ -108,12 +219,11 @@ __global__ void __launch_bounds__(kAcaThreads) r0_aca_kernel(const double *__res
       for (int j = t; j < n1; j += kAcaThreads) {
         double K[3][3];
         entry(i0, j, K);
+        aca_subtract(A + 3LL * i0, lda, Bf + 3LL * j * ldb, ldb, 3 * rank, K);
+#pragma unroll
         for (int b = 0; b < 3; b++)
-          for (int a = 0; a < 3; a++) {
-            double v = K[a][b];
-            for (int k = 0; k < 3 * rank; k++) v -= A[k * lda + 3LL * i0 + a] * Bf[(3LL * j + b) * ldb + k];
-            row[(3LL * j + b) * 3 + a] = v;
-          }
+#pragma unroll
+          for (int a = 0; a < 3; a++) row[(3LL * j + b) * 3 + a] = K[a][b];
       }
       __syncthreads();
       // pivot column block
@@ -127,9 +237,8 @@ __global__ void __launch_bounds__(kAcaThreads) r0_aca_kernel(const double *__res
           bi = j;
         }
       }
-      double gbest;
       int i1;
-      aca_argmax(best, bi, s_val, s_idx, gbest, i1);
+      aca_argmax(best, bi, s_val, s_idx, i1);
       if (i1 < 0) break;  // uniform: every thread read the same i1
       if (t == 0) {
         used0[i0] = 1;
@@ -142,12 +251,11 @@ __global__ void __launch_bounds__(kAcaThreads) r0_aca_kernel(const double *__res
       for (int i = t; i < n0; i += kAcaThreads) {
         double K[3][3];
         entry(i, i1, K);
+        aca_subtract(A + 3LL * i, lda, Bf + 3LL * i1 * ldb, ldb, 3 * rank, K);
+#pragma unroll
         for (int b = 0; b < 3; b++)
-          for (int a = 0; a < 3; a++) {
-            double v = K[a][b];
-            for (int k = 0; k < 3 * rank; k++) v -= A[k * lda + 3LL * i + a] * Bf[(3LL * i1 + b) * ldb + k];
-            A[(3LL * rank + b) * lda + 3LL * i + a] = v;
-          }
+#pragma unroll
+          for (int a = 0; a < 3; a++) A[(3LL * rank + b) * lda + 3LL * i + a] = K[a][b];
       }
       // B_k = Gamma R
       for (int j = t; j < 3 * n1; j += kAcaThreads)
@@ -158,35 +266,8 @@ __global__ void __launch_bounds__(kAcaThreads) r0_aca_kernel(const double *__res
         }
       __syncthreads();
       // |A_k B_k|_F^2 and cross terms with the earlier rank blocks
-      double part[9], ata[9], bbt[9];
-      for (int k = 0; k < 9; k++) part[k] = 0.0;
-      for (long long r = t; r < lda; r += kAcaThreads)
-        for (int a = 0; a < 3; a++)
-          for (int b = 0; b < 3; b++)
-            part[b * 3 + a] += A[(3LL * rank + a) * lda + r] * A[(3LL * rank + b) * lda + r];
-      aca_sum9(part, s_red, ata);
-      for (int k = 0; k < 9; k++) part[k] = 0.0;
-      for (long long j = t; j < 3LL * n1; j += kAcaThreads)
-        for (int a = 0; a < 3; a++)
-          for (int b = 0; b < 3; b++) part[b * 3 + a] += Bf[j * ldb + 3LL * rank + a] * Bf[j * ldb + 3LL * rank + b];
-      aca_sum9(part, s_red, bbt);
-      double ab = 0.0;
-      for (int k = 0; k < 9; k++) ab += ata[k] * bbt[k];
-      double cross = 0.0;
-      for (int r = 0; r < rank; r++) {
-        double m1[9], m2[9];
-        for (int k = 0; k < 9; k++) part[k] = 0.0;
-        for (long long q = t; q < lda; q += kAcaThreads)
-          for (int a = 0; a < 3; a++)
-            for (int b = 0; b < 3; b++) part[b * 3 + a] += A[(3LL * r + a) * lda + q] * A[(3LL * rank + b) * lda + q];
-        aca_sum9(part, s_red, m1);
-        for (int k = 0; k < 9; k++) part[k] = 0.0;
-        for (long long j = t; j < 3LL * n1; j += kAcaThreads)
-          for (int a = 0; a < 3; a++)
-            for (int b = 0; b < 3; b++) part[b * 3 + a] += Bf[j * ldb + 3LL * rank + b] * Bf[j * ldb + 3LL * r + a];
-        aca_sum9(part, s_red, m2);
-        for (int k = 0; k < 9; k++) cross += m1[k] * m2[k];
-      }
+      double ab, cross;
+      aca_frobenius(A, lda, Bf, ldb, rank, 3LL * n1, s_frob, s_sum, cross, ab);
       s_norm += 2.0 * cross + ab;
       // next row block from A_k
       best = 0.0;
@@ -203,7 +284,7 @@ __global__ void __launch_bounds__(kAcaThreads) r0_aca_kernel(const double *__res
         }
       }
       int next;
-      aca_argmax(best, bi, s_val, s_idx, gbest, next);
+      aca_argmax(best, bi, s_val, s_idx, next);
       rank++;
       if (next < 0 || rank == max_rank) break;
       if (fabs(ab) <= eps * eps * fabs(s_norm)) {

@@ -6,6 +6,7 @@
 #include <cstring>
 #include <memory>
 #include <mutex>
+#include <numeric>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -2061,12 +2062,20 @@ int bw_r0_aca(int device, int64_t n_elems, const double *records, double G, doub
     }
     if (ao > a_len || bo > b_len) throw std::invalid_argument("bw_r0_aca: factor storage smaller than the capacity");
     if (!n_lr) return BW_OK;
+    // longest first (a step's work grows with the sides, the rank with their size)
+    std::vector<int32_t> order(n_lr);
+    std::iota(order.begin(), order.end(), 0);
+    std::stable_sort(order.begin(), order.end(), [&](int32_t p, int32_t q) {
+      return blocks[p].n0 + blocks[p].n1 > blocks[q].n0 + blocks[q].n1;
+    });
+    order.push_back(0);  // the kernel's queue counter
     BW_CUDA(cudaSetDevice(device));
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int grid = (int)std::min<int64_t>(n_lr, 148 * 4);
-    void *d_rec = nullptr, *d_perm = nullptr, *d_blk = nullptr, *d_scr = nullptr, *d_rank = nullptr, *d_err = nullptr;
+    void *d_rec = nullptr, *d_perm = nullptr, *d_blk = nullptr, *d_scr = nullptr, *d_rank = nullptr, *d_err = nullptr,
+         *d_ord = nullptr;
     auto release = [&] {
-      for (void *q : {d_rec, d_perm, d_blk, d_scr, d_rank, d_err}) cudaFree(q);
+      for (void *q : {d_rec, d_perm, d_blk, d_scr, d_rank, d_err, d_ord}) cudaFree(q);
     };
     try {
       const size_t rb = sizeof(double) * bw::r0::kFrameDoubles * (size_t)n_elems;
@@ -2076,13 +2085,16 @@ int bw_r0_aca(int device, int64_t n_elems, const double *records, double G, doub
       BW_CUDA(cudaMalloc(&d_scr, sizeof(double) * (size_t)slot * grid));
       BW_CUDA(cudaMalloc(&d_rank, 4 * (size_t)n_lr));
       BW_CUDA(cudaMalloc(&d_err, 8 * (size_t)n_lr));
+      BW_CUDA(cudaMalloc(&d_ord, 4 * order.size()));
+      BW_CUDA(cudaMemcpyAsync(d_ord, order.data(), 4 * order.size(), cudaMemcpyHostToDevice, st));
       BW_CUDA(cudaMemcpyAsync(d_rec, records, rb, cudaMemcpyHostToDevice, st));
       BW_CUDA(cudaMemcpyAsync(d_perm, p32.data(), 4 * p32.size(), cudaMemcpyHostToDevice, st));
       BW_CUDA(cudaMemcpyAsync(d_blk, blocks.data(), sizeof(bw::AcaBlock) * blocks.size(), cudaMemcpyHostToDevice, st));
       bw::r0_aca_kernel<<<grid, bw::kAcaThreads, 0, st>>>(
           static_cast<const double *>(d_rec), static_cast<const int *>(d_perm),
           static_cast<const bw::AcaBlock *>(d_blk), (int)n_lr, G, nu, eps, factors_a, factors_b,
-          static_cast<double *>(d_scr), slot, static_cast<int *>(d_rank), static_cast<double *>(d_err));
+          static_cast<double *>(d_scr), slot, static_cast<const int *>(d_ord), static_cast<int *>(d_ord) + n_lr,
+          static_cast<int *>(d_rank), static_cast<double *>(d_err));
       BW_CUDA(cudaGetLastError());
       BW_CUDA(cudaMemcpyAsync(rank_out, d_rank, 4 * (size_t)n_lr, cudaMemcpyDeviceToHost, st));
       BW_CUDA(cudaMemcpyAsync(err_out, d_err, 8 * (size_t)n_lr, cudaMemcpyDeviceToHost, st));
