@@ -265,6 +265,7 @@ void build_operator(const Problem &p, bool tr, int grid, OperatorPlan &op) {
       it.h = i32(std::min<int64_t>(cut, H - r0), "item rows");
       it.hpad = i32(align_up(it.h, kRowAlign), "item rows");
       it.out_off = i32(pb[q] + r0, "output row");
+      it.panel = i32(q, "panel");
       for (int pass = 0; pass < 2; pass++) {
         for (const Cover &e : cov[q]) {
           if (e.kind != pass) continue;
@@ -701,6 +702,19 @@ void mm_chunk_item(const MmItem &it, std::vector<MmChunk> &out) {
 
 }  // namespace
 
+int mm_row_parts(int64_t panels, int64_t rows, int grid) {
+  int best = 1;
+  int64_t best_cost = -1;
+  for (int parts = 1; parts <= 8 && (parts == 1 || rows / parts >= 16); parts++) {
+    const int64_t cost = (panels * parts + grid - 1) / grid * (2 * ((rows + parts - 1) / parts) + 2 * kMmRhs);
+    if (best_cost < 0 || cost < best_cost) {
+      best = parts;
+      best_cost = cost;
+    }
+  }
+  return best;
+}
+
 void build_mm_plan(const Problem &p, bool tr, int grid, const OperatorPlan &op, MmPlan &mm) {
   mm = MmPlan{};
   mm.n_in = op.n_in;
@@ -758,8 +772,8 @@ void build_mm_plan(const Problem &p, bool tr, int grid, const OperatorPlan &op, 
       p1.items.push_back(std::move(it));
     }
   }
-  // phase 2: the matvec's row-panel items on widened windows, cut into parts
-  // of at most kMmHMax rows
+  // phase 2: the row panels on widened windows, cut into mm_row_parts equal
+  // parts (more where a part would exceed kMmHMax rows)
   MmPhase &p2 = mm.ph[1];
   auto window = [&](const Segment &sg, int64_t r0) {
     MmSeg m{};
@@ -779,12 +793,20 @@ void build_mm_plan(const Problem &p, bool tr, int grid, const OperatorPlan &op, 
     m.ncols = align_up(m.lead + m.width, 8);
     return m;
   };
-  for (const Item &src : op.ph[1].items) {
-    const int64_t parts = (src.hpad + kMmHMax - 1) / kMmHMax;
-    const int64_t cut = align_up((src.h + parts - 1) / parts, 8);
-    for (int64_t r0 = 0; r0 < src.h; r0 += cut) {
+  const std::vector<Item> &rows2 = op.ph[1].items;
+  int64_t rows_all = 0;
+  for (const Item &it : rows2) rows_all += it.h;
+  const int want_parts =
+      mm_row_parts(op.n_panels, op.n_panels > 0 ? (rows_all + op.n_panels - 1) / op.n_panels : 0, grid);
+  for (size_t q0 = 0, q1; q0 < rows2.size(); q0 = q1) {
+    const Item &src = rows2[q0];  // the panel's first item: its segments, from the panel's first row
+    int64_t H = 0;
+    for (q1 = q0; q1 < rows2.size() && rows2[q1].panel == src.panel; q1++) H += rows2[q1].h;
+    const int64_t parts = std::max<int64_t>(want_parts, (H + kMmHMax - 1) / kMmHMax);
+    const int64_t cut = align_up((H + parts - 1) / parts, 8);
+    for (int64_t r0 = 0; r0 < H; r0 += cut) {
       MmItem it;
-      it.h = i32(std::min<int64_t>(cut, src.h - r0), "item rows");
+      it.h = i32(std::min<int64_t>(cut, H - r0), "item rows");
       it.hpad = i32(align_up(it.h, 8), "item rows");
       it.out_off = i32(src.out_off + r0, "output row");
       for (const Segment &sg : src.segs) {

@@ -110,6 +110,7 @@ struct Item {
   int32_t h = 0, hpad = 0;     // rows, padded rows
   int64_t ncols = 0;           // total columns
   int32_t out_off = 0;
+  int32_t panel = -1;          // phase 2: the row panel it is (part of)
   std::vector<Segment> segs;
   std::vector<RowPiece> pieces;  // phase 1 only
 };
@@ -152,12 +153,18 @@ struct OperatorPlan {
 // worse); the queue round trip is not what limits small items.
 constexpr int kUnitBytes = 0;
 
+// The matmat's phase 1: a column of a stack brings 128 bytes of right-hand
+// sides whatever its rows, so tall items matter more than many.  64 columns,
+// 8 / 4 / 2 / 1 items: 12,288 DoF 60.8 / 58.2 / 55.5 / 56.4 us, 27,648 DoF 96.6 /
+// 90.9 / 89.4 / 91.9 us, 49,152 DoF 143.8 / 135.6 / 138.2 / 139.5 us.
+constexpr int kMmItemsPerCta = 2;
+
 // Plan parameters a tuner may change (bw_set_tuning); the defaults are the
 // compiled-in choices.
 struct Tuning {
   int items_per_cta[2] = {kItemsPerCta, kItemsPerCta};  // per phase: items per CTA share (granularity)
   int chunk_bytes = kStageBytes;                        // block data per chunk (<= kStageBytes)
-  int mm_items_per_cta = kItemsPerCta;                  // matmat phase 1
+  int mm_items_per_cta = kMmItemsPerCta;                // matmat phase 1
   int unit_bytes = kUnitBytes;                          // streaming queue: minimum cost of a unit
   int narrow_rows = 64;   // items of at most this many padded rows skip the staging (0: never) ...
   int narrow_cols = 512;  // ... warp per item up to this many columns, CTA-cooperatively above
@@ -246,7 +253,8 @@ float from_bf16(uint16_t b);
 // The phases:
 //  * phase 1: stacks of B factors per column cluster, as for the matvec, with
 //    rows on T8's numbering;
-//  * phase 2: row panels, with FR and A slices on their widened windows.
+//  * phase 2: row panels, with FR and A slices on their widened windows, cut
+//    into fewer row parts than the matvec's (mm_row_parts).
 // Block data is stored unscaled: BF16 has FP32's exponent range, so a
 // per-block scale would leave every rounded mantissa unchanged.
 constexpr int kMmRhs = 64;             // right-hand sides per pass (MMA N)
@@ -314,6 +322,16 @@ struct MmPlan {
   std::vector<MmStack> stacks;
   MmPhase ph[2];
 };
+
+// Row parts of the matmat's phase-2 panels (`panels` of `rows` rows on average,
+// `grid` CTAs).  A part streams 2 rows / parts bytes of block data and 128
+// bytes of operand per column, and an MMA covers 128 rows whether they are
+// there or not, so cutting a panel as the matvec does (24-row parts of 54-row
+// panels on a 27,648-DoF crack) multiplies the operand traffic and the MMAs.
+// Cutting pays only where it fills idle SMs: the count that takes the least
+// time, (parts of the busiest CTA) x (bytes per column).  27,648 DoF, 64
+// columns: 165 -> 106 us with the X gather's wider loads.
+int mm_row_parts(int64_t panels, int64_t rows, int grid);
 
 // Builds the matmat plan of the operator (transposed: H^T) from the problem
 // and the operator's matvec plan (its row panels are reused).

@@ -109,7 +109,7 @@ int bw_test_withhold_chunk(bw_hmat *h, int index);
  *       (granularity of the work queue), 1..256, default 8;
  *   "chunk_bytes": block data per chunk, 4096..32768, multiple of 16,
  *       default 32768;
- *   "mm_items_per_cta": granularity of the matmat's phase 1, default 8;
+ *   "mm_items_per_cta": granularity of the matmat's phase 1, default 2;
  *   "unit_bytes": the streaming queue hands out runs of consecutive items
  *       until a run's cost reaches this many bytes (0: one item at a time),
  *       0..2^30, default 0;
