@@ -3,6 +3,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstring>
 #include <memory>
 #include <mutex>
@@ -112,8 +113,10 @@ struct bw_hmat {
   std::vector<uint16_t> mm_host[2][2];  // BW_PLAN_ONLY
   uint16_t *d_xt = nullptr, *d_t8 = nullptr;  // matmat operands (8x8 BF16 tiles, bw::kMmRhs columns)
   int32_t *d_perm0 = nullptr, *d_perm1 = nullptr;
+  unsigned char *d_vectors = nullptr;  // one allocation for the vectors of a matvec:
   void *d_xp = nullptr, *d_t = nullptr, *d_g2 = nullptr;
-  void *d_xk = nullptr, *d_tk = nullptr;  // x and t of bw::kMultiMax right-hand sides, or null
+  unsigned char *d_multi = nullptr;       // scratch and run tables of several right-hand sides, or null:
+  void *d_xk = nullptr, *d_tk = nullptr;  // x and t of bw::kMultiMax of them, inside it
   double *d_xh = nullptr, *d_yh = nullptr;
   double *h_xpin = nullptr, *h_ypin = nullptr;  // pinned staging of bw_matvec_host
   cudaEvent_t y_ready[4] = {nullptr, nullptr, nullptr, nullptr};  // bw_matvec_host: output pieces landed
@@ -180,7 +183,6 @@ struct bw_hmat {
           cudaFree(ph.items);
           cudaFree(ph.queue);
           cudaFree(ph.gsegs);
-          cudaFree(ph.ranges);
           ph = DevPhase{};
         }
     for (auto &o : dmm)
@@ -196,13 +198,8 @@ struct bw_hmat {
     d_xt = d_t8 = nullptr;
     cudaFree(d_perm0);
     cudaFree(d_perm1);
-    cudaFree(d_xp);
-    cudaFree(d_t);
-    cudaFree(d_g2);
-    cudaFree(d_xk);
-    cudaFree(d_tk);
-    cudaFree(d_xh);
-    cudaFree(d_yh);
+    cudaFree(d_vectors);
+    cudaFree(d_multi);
     if (h_xpin) cudaFreeHost(h_xpin);
     if (h_ypin) cudaFreeHost(h_ypin);
     h_xpin = h_ypin = nullptr;
@@ -218,6 +215,7 @@ struct bw_hmat {
     if (stream) cudaStreamDestroy(stream);
     d_perm0 = d_perm1 = nullptr;
     d_xp = d_t = d_g2 = nullptr;
+    d_vectors = d_multi = nullptr;
     d_xk = d_tk = nullptr;
     d_xh = d_yh = nullptr;
     d_err = nullptr;
@@ -760,35 +758,35 @@ void launch_matmat_tc(bw_hmat *h, int o, const double *X, int64_t ldx, double *Y
 
 // Scratch and run tables of the FP64 / FP32 products with several right-hand
 // sides (bw_multi_kernels.cuh): 8 columns of x and t and 8 bytes per phase-2
-// chunk, about 1% of the block data.  Taken last; when they do not fit (the
-// device limit, or the device itself) such products apply one matvec per
-// column, as they do without these kernels.
+// chunk, about 1% of the block data, in one allocation.  Taken last; when it
+// does not fit (the device limit, or the device itself) such products apply
+// one matvec per column, as they do without these kernels.
 void alloc_multi(bw_hmat *h, int mask, bool with_t) {
   const int64_t es = (mask & 1) ? 8 : 4, k = bw::kMultiMax;
   if (!(mask & 3)) return;
-  std::vector<DevPhase *> made;
+  const int64_t xb = align256(std::max<int64_t>(1, std::max(h->n_rows, h->n_cols)) * k * es);
+  const int64_t tb = align256(std::max<int64_t>(1, h->sum_rank) * k * es);
+  int64_t bytes = xb + tb;
+  for (int o = 0; o < (with_t ? 2 : 1); o++)
+    for (int p = 0; p < 2; p++)
+      if (mask & (1 << p)) bytes += align256((int64_t)h->op[o].ph[1].cp[p].ranges.size() * (int64_t)sizeof(bw::RunRange));
   try {
-    for (int o = 0; o < (with_t ? 2 : 1); o++)
-      for (int p = 0; p < 2; p++) {
-        const bw::ChunkPlan &cp = h->op[o].ph[1].cp[p];
-        if (!(mask & (1 << p)) || cp.chunks.empty()) continue;
-        const auto rr = bw::run_ranges(cp);
-        static_assert(sizeof(rr[0]) == sizeof(bw::RunRange), "pairs of 32-bit integers");
-        DevPhase &dp = h->dev[o][p][1];
-        dp.ranges = static_cast<bw::RunRange *>(h->dmalloc(rr.size() * sizeof(bw::RunRange)));
-        made.push_back(&dp);
-        BW_CUDA(cudaMemcpy(dp.ranges, rr.data(), rr.size() * sizeof(bw::RunRange), cudaMemcpyHostToDevice));
-      }
-    h->d_xk = h->dmalloc((size_t)(std::max<int64_t>(1, std::max(h->n_rows, h->n_cols)) * k * es));
-    h->d_tk = h->dmalloc((size_t)(std::max<int64_t>(1, h->sum_rank) * k * es));
+    h->d_multi = static_cast<unsigned char *>(h->dmalloc((size_t)bytes));
   } catch (const OomError &) {
-    for (DevPhase *dp : made) {
-      cudaFree(dp->ranges);
-      dp->ranges = nullptr;
-    }
-    cudaFree(h->d_xk);
-    h->d_xk = nullptr;
+    return;
   }
+  h->d_xk = h->d_multi;
+  h->d_tk = h->d_multi + xb;
+  unsigned char *at = h->d_multi + xb + tb;
+  for (int o = 0; o < (with_t ? 2 : 1); o++)
+    for (int p = 0; p < 2; p++) {
+      const auto &rr = h->op[o].ph[1].cp[p].ranges;
+      if (!(mask & (1 << p)) || rr.empty()) continue;
+      static_assert(sizeof(rr[0]) == sizeof(bw::RunRange), "pairs of 32-bit integers");
+      h->dev[o][p][1].ranges = reinterpret_cast<bw::RunRange *>(at);
+      BW_CUDA(cudaMemcpy(at, rr.data(), rr.size() * sizeof(bw::RunRange), cudaMemcpyHostToDevice));
+      at += align256((int64_t)(rr.size() * sizeof(bw::RunRange)));
+    }
 }
 
 // Whether a product of several columns can run in the multi-column kernels:
@@ -1200,11 +1198,18 @@ int bw_finalize(bw_hmat *h, int flags) {
       h->d_perm1 = static_cast<int32_t *>(h->dmalloc(std::max<size_t>(1, p32.size()) * 4));
       if (!p32.empty()) BW_CUDA(cudaMemcpy(h->d_perm1, p32.data(), p32.size() * 4, cudaMemcpyHostToDevice));
       // +16 bytes: the kernels stage vector segments in 16-byte aligned windows
-      h->d_xp = h->dmalloc((size_t)std::max({xp_region_bytes(0, nmax), xp_region_bytes(2, nmax), (int64_t)1}));
-      h->d_t = h->dmalloc((size_t)std::max<int64_t>(1, h->sum_rank) * 8 + 16);
-      h->d_g2 = h->dmalloc((size_t)std::max<int64_t>(1, g2_bytes(h, mask, want_t)) + 16);
-      h->d_xh = static_cast<double *>(h->dmalloc((size_t)std::max<int64_t>(1, nmax) * 8));
-      h->d_yh = static_cast<double *>(h->dmalloc((size_t)std::max<int64_t>(1, nmax) * 8));
+      const int64_t vb[5] = {std::max({xp_region_bytes(0, nmax), xp_region_bytes(2, nmax), (int64_t)1}),
+                             std::max<int64_t>(1, h->sum_rank) * 8 + 16,
+                             std::max<int64_t>(1, g2_bytes(h, mask, want_t)) + 16,
+                             std::max<int64_t>(1, nmax) * 8, std::max<int64_t>(1, nmax) * 8};
+      int64_t vat[6] = {0};
+      for (int k = 0; k < 5; k++) vat[k + 1] = vat[k] + align256(vb[k]);
+      h->d_vectors = static_cast<unsigned char *>(h->dmalloc((size_t)vat[5]));
+      h->d_xp = h->d_vectors + vat[0];
+      h->d_t = h->d_vectors + vat[1];
+      h->d_g2 = h->d_vectors + vat[2];
+      h->d_xh = reinterpret_cast<double *>(h->d_vectors + vat[3]);
+      h->d_yh = reinterpret_cast<double *>(h->d_vectors + vat[4]);
       BW_CUDA(cudaMallocHost(&h->h_xpin, (size_t)std::max<int64_t>(1, nmax) * 8));
       BW_CUDA(cudaMallocHost(&h->h_ypin, (size_t)std::max<int64_t>(1, nmax) * 8));
       for (cudaEvent_t &e : h->y_ready) BW_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -1561,7 +1566,14 @@ int bw_plan_export(const bw_hmat *h, int precision, int phase, int transposed, i
   if (n_chunks) *n_chunks = (int64_t)cp.chunks.size();
   if (n_elems) *n_elems = ph.n_elems[p];
   if (n_item_ptr) *n_item_ptr = (int64_t)cp.item_ptr.size();
-  if (chunks) std::memcpy(chunks, cp.chunks.data(), cp.chunks.size() * sizeof(Chunk));  // kChunkWords int32 each
+  if (chunks) {
+    std::memcpy(chunks, cp.chunks.data(), cp.chunks.size() * sizeof(Chunk));  // kChunkWords int32 each
+    if (phase == 2) {
+      const std::vector<int32_t> g_off = bw::slice_per_chunk(cp).g_off;
+      for (size_t i = 0; i < g_off.size(); i++)
+        std::memcpy(chunks + i * bw::kChunkWords + offsetof(Chunk, g_off) / 4, &g_off[i], 4);
+    }
+  }
   if (item_ptr) std::memcpy(item_ptr, cp.item_ptr.data(), cp.item_ptr.size() * sizeof(int32_t));
   if (data) {
     if (!h->plan_only) return BW_ERR_STATE;
@@ -1673,7 +1685,7 @@ int bw_plan_gather(const bw_hmat *h, int precision, int transposed, int64_t *n, 
   if (p < 0 || !h->finalized || !(h->stored & (1 << p))) return BW_ERR_STATE;
   const int o = transposed ? 1 : 0;
   if (o == 1 && !h->has_t) return BW_ERR_UNSUPPORTED;
-  const std::vector<bw::GatherSeg> &g = h->op[o].ph[1].cp[p].gsegs;
+  const std::vector<bw::GatherSeg> g = bw::slice_per_chunk(h->op[o].ph[1].cp[p]).gsegs;
   *n = (int64_t)g.size();
   if (runs) std::memcpy(runs, g.data(), g.size() * sizeof(bw::GatherSeg));
   return BW_OK;

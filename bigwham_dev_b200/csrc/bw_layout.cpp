@@ -84,6 +84,12 @@ EffLow eff_low(const Problem &p, bool tr, size_t k) {
 
 int64_t align_up(int64_t v, int64_t a) { return (v + a - 1) / a * a; }
 
+// Most entries of one item of a phase.
+int64_t item_cap(int64_t entries, int64_t grid, int items_per_cta) {
+  if (items_per_cta <= 0) items_per_cta = entries / grid < kSmallShare ? kItemsPerCtaSmall : kItemsPerCta;
+  return std::max<int64_t>(1, entries / grid / items_per_cta);
+}
+
 }  // namespace
 
 void build_operator(const Problem &p, bool tr, int grid, OperatorPlan &op) {
@@ -131,7 +137,7 @@ void build_operator(const Problem &p, bool tr, int grid, OperatorPlan &op) {
   grid = std::max(1, grid);
   int64_t e1 = 0;  // phase-1 entries
   for (size_t k = 0; k < nlr; k++) e1 += p.lr[k].r * eff_low(p, tr, k).n;
-  const int64_t cap1 = std::max<int64_t>(1, e1 / grid / std::max(1, p.tune.items_per_cta[0]));
+  const int64_t cap1 = item_cap(e1, grid, p.tune.items_per_cta[0]);
   PhasePlan &p1 = op.ph[0];
   for (auto &kv : stacks) {
     const int64_t j0 = kv.first.first, n = kv.first.second;
@@ -254,7 +260,7 @@ void build_operator(const Problem &p, bool tr, int grid, OperatorPlan &op) {
     for (const Cover &e : cov[q]) pw[q] += e.kind == 0 ? e.n : eff_low(p, tr, e.k).r;
     e2 += pw[q] * (pb[q + 1] - pb[q]);
   }
-  const int64_t cap2 = std::max<int64_t>(1, e2 / grid / std::max(1, p.tune.items_per_cta[1]));
+  const int64_t cap2 = item_cap(e2, grid, p.tune.items_per_cta[1]);
   for (size_t q = 0; q < npan; q++) {
     const int64_t H = pb[q + 1] - pb[q];
     int64_t parts = 1;
@@ -379,7 +385,7 @@ float seg_scale(const OperatorPlan &op, const Segment &s, int prec) {
 // Chunks of one item for one precision; phase-2 chunks also get their slice of
 // the gather array (g_len grows) and the runs that fill it.
 void chunk_item(const OperatorPlan &op, const Item &it, int prec, int phase, int chunk_bytes, std::vector<Chunk> &out,
-                std::vector<GatherSeg> &gsegs, int64_t &g_len) {
+                std::vector<std::pair<int32_t, int32_t>> &ranges, std::vector<GatherSeg> &gsegs, int64_t &g_len) {
   const int es = esize_of(prec);
   const bool tiled = prec == 2;
   int64_t cap;
@@ -404,6 +410,7 @@ void chunk_item(const OperatorPlan &op, const Item &it, int prec, int phase, int
     if (phase == 0) {
       ch.g_off = it.segs.empty() ? 0 : i32(it.segs[0].src_off + c0, "vector offset");
     } else {
+      const size_t first = gsegs.size();
       const int64_t g = (g_len + 3) / 4 * 4;  // 16-byte aligned slice in FP32, 32 in FP64
       if (g + take > INT32_MAX) throw std::runtime_error("gather array above 2^31 entries");
       ch.g_off = i32(g, "G2 offset");
@@ -420,6 +427,7 @@ void chunk_item(const OperatorPlan &op, const Item &it, int prec, int phase, int
         gs.scale = seg_scale(op, sg, prec);
         gsegs.push_back(gs);
       }
+      ranges.emplace_back(i32((int64_t)first, "run"), i32((int64_t)(gsegs.size() - first), "run count"));
     }
     if (out.empty()) ch.flags |= kFirst;
     c0 += take;
@@ -445,10 +453,28 @@ void build_chunks(const Problem &p, bool tr, int prec, int grid, OperatorPlan &o
     }
     ph.n_elems[prec] = off + kItemAlign;  // slack so 16-byte rounded copies stay inside
     std::vector<std::vector<Chunk>> per_item(ph.items.size());
+    std::vector<std::vector<std::pair<int32_t, int32_t>>> runs_of(ph.items.size());
     cp.gsegs.clear();
     cp.g_len = 0;
-    for (size_t q = 0; q < ph.items.size(); q++)
-      chunk_item(op, ph.items[q], prec, phase, p.tune.chunk_bytes, per_item[q], cp.gsegs, cp.g_len);
+    for (size_t q = 0, q0 = 0; q < ph.items.size(); q++) {
+      const Item &it = ph.items[q];
+      if (q > 0 && it.panel != ph.items[q - 1].panel) q0 = q;
+      // an earlier part of the same panel and height has the same cuts: its
+      // slices of G2 serve this part too
+      size_t like = q0;
+      while (phase == 1 && like < q && ph.items[like].hpad != it.hpad) like++;
+      if (phase == 0 || like == q) {
+        chunk_item(op, it, prec, phase, p.tune.chunk_bytes, per_item[q], runs_of[q], cp.gsegs, cp.g_len);
+        continue;
+      }
+      per_item[q] = per_item[like];
+      runs_of[q] = runs_of[like];
+      for (Chunk &c : per_item[q]) {
+        c.data_off += it.off[prec] - ph.items[like].off[prec];
+        c.rows = it.h;
+        c.out_off = it.out_off;
+      }
+    }
     // Longest first: the CTAs take items from a queue in this order (greedy
     // list scheduling; each CTA takes the next item when its producer is
     // done with the previous one).  Cost is the bytes streamed plus a fixed
@@ -465,11 +491,13 @@ void build_chunks(const Problem &p, bool tr, int prec, int grid, OperatorPlan &o
     // walks a unit's chunks as one range; item boundaries stay in the chunk
     // flags, so results do not depend on the grouping.
     cp.chunks.clear();
+    cp.ranges.clear();
     cp.item_ptr.assign(1, 0);
     int64_t unit_cost = 0;
     for (size_t k = 0; k < order.size(); k++) {
       const int64_t q = order[k];
       cp.chunks.insert(cp.chunks.end(), per_item[q].begin(), per_item[q].end());
+      cp.ranges.insert(cp.ranges.end(), runs_of[q].begin(), runs_of[q].end());
       if (cp.chunks.size() > (size_t)INT32_MAX) fail("too many chunks");
       unit_cost += cost[q];
       if (unit_cost >= p.tune.unit_bytes || k + 1 == order.size()) {
@@ -480,19 +508,18 @@ void build_chunks(const Problem &p, bool tr, int prec, int grid, OperatorPlan &o
   }
 }
 
-std::vector<std::pair<int32_t, int32_t>> run_ranges(const ChunkPlan &cp) {
-  // the runs are made chunk by chunk, so their places in G2 increase
-  std::vector<std::pair<int32_t, int32_t>> out;
-  out.reserve(cp.chunks.size());
-  for (const Chunk &c : cp.chunks) {
-    auto it = std::lower_bound(cp.gsegs.begin(), cp.gsegs.end(), c.g_off,
-                               [](const GatherSeg &g, int32_t at) { return g.dst < at; });
-    const int64_t first = it - cp.gsegs.begin();
-    int64_t count = 0, cols = 0;
-    for (; cols < c.ncols && it != cp.gsegs.end() && it->dst == c.g_off + cols; ++it, count++)
-      cols += it->cols_src & 0x7fffffffu;
-    if (cols != c.ncols) fail("the runs of a chunk do not tile its vector values");
-    out.emplace_back(i32(first, "run"), i32(count, "run count"));
+ChunkSlices slice_per_chunk(const ChunkPlan &cp) {
+  ChunkSlices out;
+  int64_t len = 0;
+  for (size_t i = 0; i < cp.ranges.size(); i++) {
+    const int64_t g = (len + 3) / 4 * 4;
+    out.g_off.push_back(i32(g, "G2 offset"));
+    for (int32_t k = 0; k < cp.ranges[i].second; k++) {
+      GatherSeg s = cp.gsegs[cp.ranges[i].first + k];
+      s.dst = i32(g + (s.dst - cp.chunks[i].g_off), "G2 offset");
+      out.gsegs.push_back(s);
+    }
+    len = g + cp.chunks[i].ncols;
   }
   return out;
 }

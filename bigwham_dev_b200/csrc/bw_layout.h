@@ -38,7 +38,14 @@ constexpr int kMaxColsFp64 = 256;    // FP64 chunks (items of 8 rows would reach
 constexpr int kHMax = 512;           // max padded rows of one item
 constexpr int kRowAlign = 8;         // padded rows are a multiple of this
 constexpr int kItemAlign = 64;       // item start alignment, in elements
-constexpr int kItemsPerCta = 8;      // minimum items per CTA share (load balance)
+// Minimum items per CTA share (load balance) when the tuning names none: 4, and
+// 8 for a phase of less than kSmallShare entries per CTA, whose few items are
+// else too uneven.  Matvec at 4 / 8 items: 3DR0 FP32 3,600 DoF 44.9 / 34.9 us,
+// 27,648 DoF 111 / 125 us, 49,152 DoF 185 / 189 us (BF16 142 / 156 us), 196,608
+// DoF 888 / 888 us; 3DT0 BF16 132,150 DoF 289 / 313 us.
+constexpr int kItemsPerCta = 4;
+constexpr int kItemsPerCtaSmall = 8;
+constexpr int64_t kSmallShare = 32768;
 
 // Chunk flags
 constexpr uint32_t kFirst = 1u;      // first chunk of an item: reset accumulators
@@ -123,8 +130,21 @@ struct ChunkPlan {
   std::vector<Chunk> chunks;
   std::vector<int32_t> item_ptr;  // queue units + 1 (chunk index of each unit's first chunk)
   std::vector<GatherSeg> gsegs;   // phase 2 only
+  // phase 2: each chunk's runs in gsegs (first, count), in the chunks' order;
+  // they tile the chunk's vector values in order
+  std::vector<std::pair<int32_t, int32_t>> ranges;
   int64_t g_len = 0;
 };
+
+// A phase-2 plan with a slice of G2 for every chunk, as the plan export shows
+// it.  The plan itself shares: the row parts of one panel multiply the same
+// vector values, and those of equal height are cut into the same columns, so
+// they read one slice.
+struct ChunkSlices {
+  std::vector<int32_t> g_off;     // per chunk
+  std::vector<GatherSeg> gsegs;
+};
+ChunkSlices slice_per_chunk(const ChunkPlan &cp);
 
 struct PhasePlan {
   std::vector<Item> items;
@@ -162,7 +182,7 @@ constexpr int kMmItemsPerCta = 2;
 // Plan parameters a tuner may change (bw_set_tuning); the defaults are the
 // compiled-in choices.
 struct Tuning {
-  int items_per_cta[2] = {kItemsPerCta, kItemsPerCta};  // per phase: items per CTA share (granularity)
+  int items_per_cta[2] = {0, 0};  // per phase: items per CTA share (granularity; 0: by size, kItemsPerCta)
   int chunk_bytes = kStageBytes;                        // block data per chunk (<= kStageBytes)
   int mm_items_per_cta = kMmItemsPerCta;                // matmat phase 1
   int unit_bytes = kUnitBytes;                          // streaming queue: minimum cost of a unit
@@ -192,7 +212,7 @@ struct Problem {
 // Validates the pattern and builds the structural plan (items) of the operator
 // (transposed = true builds H^T from the same blocks).  Throws std::runtime_error
 // with a message on a malformed pattern.
-// Items are cut so that none holds more than 1/kItemsPerCta of the average
+// Items are cut so that none holds more than 1/items_per_cta of the average
 // per-CTA share of `grid` CTAs (static scheduling needs fine grains).
 void build_operator(const Problem &p, bool transposed, int grid, OperatorPlan &op);
 
@@ -204,11 +224,6 @@ void compute_scales(const Problem &p, bool transposed, bool check_finite, Operat
 // into chunks, and orders the items longest first (cost = bytes + a per-chunk
 // overhead): the kernel's CTAs take them in that order from a device queue.
 void build_chunks(const Problem &p, bool transposed, int prec, int grid, OperatorPlan &op);
-
-// Each chunk's runs in a phase-2 plan's run list, in the chunks' order: (first
-// run, number of runs).  The runs of a chunk are consecutive and tile its slice
-// of the vector values in order (std::runtime_error otherwise).
-std::vector<std::pair<int32_t, int32_t>> run_ranges(const ChunkPlan &cp);
 
 // Writes the data of items [i_begin, i_end) of one phase, converted to the
 // precision and in its layout, into dst (dst[0] is element `base` of the

@@ -106,7 +106,8 @@ int bw_test_withhold_chunk(bw_hmat *h, int index);
 /* Plan parameters, set before bw_finalize (bigwham_dev_b200/tune.py sweeps
  * them on a GPU and commits the best per workload):
  *   "items_per_cta_phase1", "items_per_cta_phase2": items per CTA share
- *       (granularity of the work queue), 1..256, default 8;
+ *       (granularity of the work queue), 1..256, default 4, or 8 for a phase
+ *       of less than 32,768 entries per CTA;
  *   "chunk_bytes": block data per chunk, 4096..32768, multiple of 16,
  *       default 32768;
  *   "mm_items_per_cta": granularity of the matmat's phase 1, default 2;
@@ -267,8 +268,10 @@ int bw_mm_plan_export(const bw_hmat *h, int phase, int transposed, int64_t *n_ch
  * converted to double, in the precision's layout (column-major items for FP64 /
  * FP32, 8x8 tiles for BF16; BF16 values divided by their block scale);
  * item_ptr: the chunk ranges of the items (n_item_ptr = items + 1 offsets), in
- * the order the kernel's CTAs take them (longest first).  data is only
- * available on a handle finalized with BW_PLAN_ONLY. */
+ * the order the kernel's CTAs take them (longest first).  Phase 2 is shown with
+ * a slice of the gather array for every chunk; on the device the row parts of
+ * one panel share theirs.  data is only available on a handle finalized with
+ * BW_PLAN_ONLY. */
 int bw_plan_export(const bw_hmat *h, int precision, int phase, int transposed, int64_t *n_chunks,
                    int32_t *chunks, int64_t *n_elems, double *data, int64_t *n_item_ptr, int32_t *item_ptr);
 
