@@ -473,7 +473,7 @@ void pack_phase_device(bw_hmat *h, int o, int prec, int phase, void *dst) {
 // kernel the rest, warp per unit.  narrow_coop 1: the CTA-wide kernel only
 // up to the last tall unit, the unstaged kernel's CTAs take the long ones
 // after it whole (units [wide, coop)).  narrow_rows 0: everything CTA-wide.
-bw::NarrowSplit narrow_split(const bw::ChunkPlan &cp, const bw::Tuning &tune) {
+bw::NarrowSplit narrow_split(const bw::ChunkPlan &cp, const bw::Tuning &tune, int grid) {
   const int64_t n_units = std::max<int64_t>(0, (int64_t)cp.item_ptr.size() - 1);
   bw::NarrowSplit sp{n_units, n_units};
   if (tune.narrow_rows <= 0) return sp;
@@ -493,6 +493,10 @@ bw::NarrowSplit narrow_split(const bw::ChunkPlan &cp, const bw::Tuning &tune) {
     sp.coop = std::max(sp.wide, last_long + 1);
   } else {
     sp.wide = std::max(last_tall, last_long) + 1;
+    // A few units left over: the CTA-wide launch that fills the chip anyway
+    // takes them with the rest (3DR0 FP64, 12,288 DoF: 16 of phase 1's 1,355
+    // units in a launch of their own took 22 us; matvec 112 -> 90 us).
+    if (sp.wide >= grid && 4 * (n_units - sp.wide) <= sp.wide) sp.wide = n_units;
     sp.coop = sp.wide;
   }
   return sp;
@@ -508,7 +512,7 @@ void upload_phase(bw_hmat *h, int o, int prec, int phase) {
   const bw::ChunkPlan &cp = ph.cp[prec];
   dp.n_chunks = (int64_t)cp.chunks.size();
   dp.n_gsegs = (int64_t)cp.gsegs.size();
-  dp.split = narrow_split(cp, h->prob.tune);
+  dp.split = narrow_split(cp, h->prob.tune, h->grid);
   if (h->plan_only) {
     auto &buf = h->host_data[o][prec][phase];
     buf.assign((size_t)ph.n_elems[prec] * es, 0);
@@ -583,6 +587,23 @@ void compute_diagonal(bw_hmat *h) {
   }
 }
 
+// A launch that may start before the one in front of it on the stream has
+// finished (`early`; the kernel then waits where it needs that one's results).
+template <typename... P, typename... A>
+void launch(void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t st, bool early, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = early ? 1 : 0;
+  BW_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+}
+
 // The launches of one matvec: x gather (+ permutation), phase 1 (t), G2
 // gather, phase 2 (y), each phase in the CTA-wide and / or the unstaged
 // kernel, with the given scratch vectors; `ev` (optional) receives
@@ -648,19 +669,11 @@ void launch_matvec_impl(bw_hmat *h, int o, int prec, const double *x, double *y,
         a.n_items = (int)(dp.n_items - dp.split.wide);
         a.n_coop = (int)(dp.split.coop - dp.split.wide);
         a.queue = dp.queue + 2;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(2 * h->grid);
-        cfg.blockDim = dim3(32 * bw::kNarrowWarps);
-        cfg.dynamicSmemBytes = 0;
-        cfg.stream = st;
-        // After the phase's CTA-wide launch (and no timing event between
-        // them) it may start on the SMs that launch leaves free or frees.
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = (dp.split.wide > 0 && !ev) ? 1 : 0;
-        BW_CUDA(cudaLaunchKernelEx(&cfg, bw::narrow_items_kernel<S>, a));
+        a.team = bw::narrow_team(dp.n_items - dp.split.coop, h->grid);
+        // after the phase's CTA-wide launch (and no timing event between them)
+        // it may start on the SMs that launch leaves free or frees
+        launch(a.team > 1 ? bw::narrow_items_kernel<S, true> : bw::narrow_items_kernel<S, false>, 2 * h->grid,
+               32 * bw::kNarrowWarps, 0, st, dp.split.wide > 0 && !ev, a);
       }
     }
     if (ev) {
@@ -839,23 +852,14 @@ void launch_multi(bw_hmat *h, int o, int prec, const double *X, int64_t ldx, dou
     m.nrhs = nrhs;
     if (dp.split.wide > 0) {
       m.s.n_items = (int)dp.split.wide;
-      bw::stream_multi_kernel<S, K><<<h->grid, bw::threads_of<S>(), L::kTotal, st>>>(m);
-      BW_CUDA(cudaGetLastError());
+      launch(bw::stream_multi_kernel<S, K>, h->grid, bw::threads_of<S>(), L::kTotal, st, false, m);
     }
     if (dp.split.wide < dp.n_items) {
       m.s.item_ptr = dp.items + dp.split.wide;
       m.s.n_items = (int)(dp.n_items - dp.split.wide);
       m.s.queue = dp.queue + 2;
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(2 * h->grid);
-      cfg.blockDim = dim3(32 * bw::kMultiNarrowWarps);
-      cfg.stream = st;
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-      attr[0].val.programmaticStreamSerializationAllowed = 1;
-      cfg.attrs = attr;
-      cfg.numAttrs = dp.split.wide > 0 ? 1 : 0;
-      BW_CUDA(cudaLaunchKernelEx(&cfg, bw::narrow_multi_kernel<S, K>, m));
+      m.s.team = bw::narrow_team(dp.n_items - dp.split.wide, h->grid);
+      launch(bw::narrow_multi_kernel<S, K>, h->grid, 32 * bw::kNarrowWarps, 0, st, dp.split.wide > 0, m);
     }
   }
 }
@@ -1596,7 +1600,7 @@ int bw_plan_split(const bw_hmat *h, int precision, int phase, int transposed, in
   if (p < 0 || !h->finalized || !(h->stored & (1 << p))) return BW_ERR_STATE;
   const int o = transposed ? 1 : 0;
   if (o == 1 && !h->has_t) return BW_ERR_UNSUPPORTED;
-  const bw::NarrowSplit sp = narrow_split(h->op[o].ph[phase - 1].cp[p], h->prob.tune);
+  const bw::NarrowSplit sp = narrow_split(h->op[o].ph[phase - 1].cp[p], h->prob.tune, h->grid);
   *n_wide = sp.wide;
   *n_coop = sp.coop;
   return BW_OK;
@@ -1614,7 +1618,7 @@ int bw_matvec_launches(const bw_hmat *h, int precision, int transposed, int64_t 
     const int64_t units = std::max<int64_t>(0, (int64_t)cp.item_ptr.size() - 1);
     if (ph == 1 && !cp.gsegs.empty()) k++;  // G2 gather
     if (cp.chunks.empty()) continue;
-    const bw::NarrowSplit sp = narrow_split(cp, h->prob.tune);
+    const bw::NarrowSplit sp = narrow_split(cp, h->prob.tune, h->grid);
     k += (sp.wide > 0 ? 1 : 0) + (sp.wide < units ? 1 : 0);
   }
   *n = k;

@@ -50,7 +50,8 @@ struct StreamArgs {
   const Chunk *chunks;        // item by item
   const int32_t *item_ptr;    // chunk ranges of the items, longest first (n_items + 1)
   int n_items;
-  int n_coop;                 // warp-per-item kernel: units [0, n_coop) run CTA-cooperatively
+  int n_coop;                 // unstaged kernel: units [0, n_coop) run CTA-cooperatively
+  int team;                   // unstaged kernel: warps per unit for the rest (1, 2, 4, 8 or 16)
   int *queue;                 // [next item, CTAs done(, next CTA-cooperative unit)]: zero at launch, reset
                               // to zero by the last CTA
   const void *gsrc;           // vector values: gathered x (phase 1) or G2 (phase 2), compute type
@@ -123,6 +124,11 @@ __device__ __forceinline__ void pdl_launch_dependents() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Barrier `id` (1..15) over the `threads` threads that use it.
+__device__ __forceinline__ void bar_sync(int id, int threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
 
 __device__ __forceinline__ void fence_barrier_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -524,7 +530,8 @@ __global__ void __launch_bounds__(threads_of<S>(), 1) stream_panels_kernel(Strea
 #pragma unroll
   for (int r = 0; r < R; r++) acc[r] = 0;
   // tensor path state
-  int nMt = 1, kparts = 1, mg = 0, kp = 0;
+  int nMt = 1, kparts = 1, kp = 0;
+  int mt0 = 0, njt = 0;  // this warp's m-tiles: mt0 .. mt0 + njt - 1
   int rot = 0;  // rotation of the K-step deal: chunk index within the item, mod kparts
   bool wact = false;
   float tacc[kTensor ? 8 : 1][4];
@@ -583,11 +590,16 @@ __global__ void __launch_bounds__(threads_of<S>(), 1) stream_panels_kernel(Strea
     } else {
       if (flags & kFirst) {
         nMt = (hpad + 15) >> 4;
+        // groups of at most 8 m-tiles, of even size: 9 tiles go 5 + 4 (8 + 1
+        // leaves half the warps with an eighth of the work; the 72-row halves
+        // of 129-row panels, 5 tiles, were the faster cut before)
         const int mgroups = (nMt + 7) >> 3;
         kparts = kConsumerWarps / mgroups;
-        mg = cw / kparts;
+        const int mg = cw / kparts;
         kp = cw % kparts;
         wact = mg < mgroups;
+        mt0 = mg * nMt / mgroups;
+        njt = (mg + 1) * nMt / mgroups - mt0;
         rot = 0;
 #pragma unroll
         for (int j = 0; j < 8; j++)
@@ -649,7 +661,7 @@ __global__ void __launch_bounds__(threads_of<S>(), 1) stream_panels_kernel(Strea
             const uint32_t kaddr = lane_base + static_cast<uint32_t>(ks) * kstep_bytes - (k2 ? 0u : back_k);
 #pragma unroll
             for (int j = 0; j < kNJ; j++) {
-              const int mt = mg * 8 + j;
+              const int mt = mt0 + j;
               const bool m2 = mt != half_mt;  // second 8-row group present
               uint32_t a0, a1, a2, a3;
               ldmatrix_x4_trans(kaddr + 256u * static_cast<uint32_t>(mt) - (m2 ? 0u : back_m), a0, a1, a2, a3);
@@ -665,7 +677,7 @@ __global__ void __launch_bounds__(threads_of<S>(), 1) stream_panels_kernel(Strea
             }
           }
         };
-        switch (min(8, nMt - mg * 8)) {
+        switch (njt) {
           case 1: ksteps(IntC<1>{}); break;
           case 2: ksteps(IntC<2>{}); break;
           case 3: ksteps(IntC<3>{}); break;
@@ -694,8 +706,8 @@ __global__ void __launch_bounds__(threads_of<S>(), 1) stream_panels_kernel(Strea
           const int g8 = lane >> 2;
 #pragma unroll
           for (int j = 0; j < 8; j++) {
-            const int mt = mg * 8 + j;
-            if (mt < nMt) {
+            const int mt = mt0 + j;
+            if (j < njt) {
               const int row = mt * 16 + g8;
               if (row < hpad) rb[kp * hpad + row] = tacc[j][0] + tacc[j][1];
               if (row + 8 < hpad) rb[kp * hpad + row + 8] = tacc[j][2] + tacc[j][3];
@@ -739,8 +751,10 @@ __global__ void __launch_bounds__(threads_of<S>(), 1) stream_panels_kernel(Strea
 //     with the narrow_coop tuning, by default those stay in the CTA-wide
 //     kernel): the CTA's 16 warps take the unit's chunks round robin, and the
 //     warps' rows of each item are added in shared memory, in warp order;
-//   * warp per unit (the rest): a warp takes a unit from the queue and writes
-//     its outputs itself; nothing is shared between warps.
+//   * the rest: with many units, a warp takes a unit from the queue and writes
+//     its outputs itself; with few (small matrices, a phase's last items), a
+//     team of 2 to 16 warps shares a unit's columns, so that the warps of the
+//     chip are used whatever the number of units (narrow_team).
 // After a CTA-wide launch of the same phase it runs as that launch's
 // programmatic dependent (pdl_launch_dependents / pdl_wait).
 // A warp walks a chunk in rounds: each lane issues all of a round's loads
@@ -751,6 +765,16 @@ __global__ void __launch_bounds__(threads_of<S>(), 1) stream_panels_kernel(Strea
 // or CTA that takes it.
 constexpr int kNarrowRows = 64;
 constexpr int kNarrowWarps = 16;  // per CTA; two CTAs per SM
+
+// Warps per unit: the most that leave every unit a team of its own among the
+// resident warps (2 CTAs per SM).  One warp streams about 3 bytes/ns whatever
+// the rest of the chip does, so 32 units of 29 KB (a 256-segment crack's
+// phase 2) took 13 us with a warp each; its matvec 34.0 -> 25.7 us.
+inline int narrow_team(long long units, int sms) {
+  int team = kNarrowWarps;
+  while (team > 1 && units * team > 2LL * sms * kNarrowWarps) team >>= 1;
+  return team;
+}
 
 // x value of a packed (hi, lo) BF16 word (pack_hilo): hi + lo, exact in FP32.
 __device__ __forceinline__ float unpack_hilo(uint32_t w) {
@@ -766,19 +790,21 @@ __device__ __forceinline__ int narrow_lpc(int hpad, int R) {
   return lpc;
 }
 
-// One chunk of a column-major FP64 / FP32 item: lane (slot, r0) takes columns
-// slot, slot + cpp, ... in rounds of kAhead.
+// One chunk of a column-major FP64 / FP32 item: lane (slot, r0) of warp tw of
+// the unit's `team` takes columns slot + cpp tw, + cpp team, ... in rounds of
+// kAhead.
 template <typename S, int R>
 __device__ __forceinline__ void narrow_fma_chunk(const unsigned char *base, const typename Store<S>::G *g, int hpad,
-                                                 int ncols, int lpc, int lane, typename Store<S>::G (&acc)[R]) {
+                                                 int ncols, int lpc, int lane, int tw, int team,
+                                                 typename Store<S>::G (&acc)[R]) {
   using G = typename Store<S>::G;
   using V = typename std::conditional<sizeof(G) == 8, double2, float4>::type;
   constexpr int kAhead = sizeof(G) == 8 ? 4 : 6;  // 16-byte loads in flight per lane
-  const int r0 = (lane % lpc) * R, cpp = 32 / lpc;
+  const int r0 = (lane % lpc) * R, cpp = (32 / lpc) * team;
   if (r0 >= hpad) return;
   const G *d = reinterpret_cast<const G *>(base) + r0;
 #pragma unroll 1
-  for (int c = lane / lpc; c < ncols; c += kAhead * cpp) {
+  for (int c = lane / lpc + (32 / lpc) * tw; c < ncols; c += kAhead * cpp) {
     V v[kAhead];
     G x[kAhead];
 #pragma unroll
@@ -812,22 +838,23 @@ __device__ __forceinline__ int narrow_rgl(int hpad) {
   return nrg <= 1 ? 1 : nrg <= 2 ? 2 : 4;
 }
 
-// One chunk of an 8x8-tiled BF16 item: lane (c8, rl, cs) takes column groups
-// cs, cs + gpw, ... in rounds of kAhead.  Items of at most 4 row groups load
+// One chunk of an 8x8-tiled BF16 item: lane (c8, rl, cs) of warp tw of the
+// unit's `team` takes column groups cs + gpw tw, + gpw team, ... in rounds of
+// kAhead.  Items of at most 4 row groups load
 // one tile column per lane and column group (four column groups a round),
 // items of 5 to 8 row groups two (two a round).
 template <bool kTwo>
 __device__ __forceinline__ void narrow_bf16_chunk_t(const uint16_t *base, const uint32_t *g, int hpad, int ncols,
-                                                    int lane, float (&acc)[2][8]) {
+                                                    int lane, int tw, int team, float (&acc)[2][8]) {
   constexpr int kAhead = kTwo ? 2 : 4;
-  const int nrg = hpad >> 3, rgl = narrow_rgl(hpad), gpw = 4 / rgl;
+  const int nrg = hpad >> 3, rgl = narrow_rgl(hpad), gpw = (4 / rgl) * team;
   const int c8 = lane & 7, rl = (lane >> 3) & (rgl - 1), cs = (lane >> 3) / rgl;
   const int ncg = (ncols + 7) >> 3;
   const bool one = rl < nrg;               // no row group 3 when nrg = 3
   const bool two = kTwo && rl + 4 < nrg;  // a second row group
   const uint16_t *lb = base + c8 * 8 + rl * 64;
 #pragma unroll 1
-  for (int cg = cs; cg < ncg; cg += kAhead * gpw) {
+  for (int cg = cs + (4 / rgl) * tw; cg < ncg; cg += kAhead * gpw) {
     float x[kAhead];
     uint4 w[kAhead][kTwo ? 2 : 1];
 #pragma unroll
@@ -929,19 +956,20 @@ struct NarrowAcc {
 #pragma unroll
       for (int k = 0; k < 8; k++) tacc[j][k] = 0.f;
   }
-  __device__ __forceinline__ void add_chunk(const StreamArgs &a, const NarrowChunk &d, int lane) {
+  __device__ __forceinline__ void add_chunk(const StreamArgs &a, const NarrowChunk &d, int lane, int tw = 0,
+                                            int team = 1) {
     using G = typename Store<S>::G;
     const unsigned char *gdata = static_cast<const unsigned char *>(a.data);
     if constexpr (kTensor) {
       const uint16_t *base = reinterpret_cast<const uint16_t *>(gdata) + d.data_off;
       const uint32_t *g = static_cast<const uint32_t *>(a.gsrc) + d.g_off;
       if (d.hpad > 32)
-        narrow_bf16_chunk_t<true>(base, g, d.hpad, d.ncols, lane, tacc);
+        narrow_bf16_chunk_t<true>(base, g, d.hpad, d.ncols, lane, tw, team, tacc);
       else
-        narrow_bf16_chunk_t<false>(base, g, d.hpad, d.ncols, lane, tacc);
+        narrow_bf16_chunk_t<false>(base, g, d.hpad, d.ncols, lane, tw, team, tacc);
     } else {
       narrow_fma_chunk<S, R>(gdata + d.data_off * Store<S>::kEsize, static_cast<const G *>(a.gsrc) + d.g_off, d.hpad,
-                             d.ncols, narrow_lpc(d.hpad, R), lane, acc);
+                             d.ncols, narrow_lpc(d.hpad, R), lane, tw, team, acc);
     }
   }
   // The item's rows summed over the warp's lanes; f(r, value) for every row
@@ -988,6 +1016,32 @@ __device__ __forceinline__ void narrow_unit_warp(const StreamArgs &a, int cb, in
   }
 }
 
+// Team per unit: the team's warps share every chunk's columns; at an item's
+// last chunk their rows meet in red (kNarrowWarps x kNarrowRows) and are summed
+// in warp order.
+template <typename S>
+__device__ __forceinline__ void narrow_unit_team(const StreamArgs &a, int cb, int ce, int lane, int wid, int team,
+                                                 typename Store<S>::G *red) {
+  using G = typename Store<S>::G;
+  const int tw = wid & (team - 1), w0 = wid - tw, bar = 1 + wid / team;
+  NarrowAcc<S> ac;
+  for (int i = cb; i < ce; i++) {
+    const NarrowChunk d = narrow_desc(a, i, tw == 0 && lane == 0);
+    if (d.flags & kFirst) ac.zero();
+    ac.add_chunk(a, d, lane, tw, team);
+    if (d.flags & kLast) {
+      ac.rows(d.hpad, lane, [&](int r, G v) { red[wid * kNarrowRows + r] = v; });
+      bar_sync(bar, 32 * team);
+      for (int r = 32 * tw + lane; r < d.rows; r += 32 * team) {
+        G sum = red[w0 * kNarrowRows + r];
+        for (int w = 1; w < team; w++) sum += red[(w0 + w) * kNarrowRows + r];
+        narrow_store<G>(a, d.out_off, r, sum);
+      }
+      bar_sync(bar, 32 * team);
+    }
+  }
+}
+
 // CTA per unit: item by item, warp w takes the item's chunks w, w + 16, ...,
 // then the warps' rows meet in red (kNarrowWarps x kNarrowRows) and are summed
 // in warp order.  Every thread of the CTA calls it.
@@ -1019,11 +1073,14 @@ __device__ __forceinline__ void narrow_unit_cta(const StreamArgs &a, int cb, int
   }
 }
 
-template <typename S>
+// kTeam: teams of warps (a.team > 1); a warp per unit otherwise, in a kernel of
+// its own: with both in one the BF16 loops spill (48-crack batch 137 -> 145 us).
+template <typename S, bool kTeam>
 __global__ void __launch_bounds__(32 * kNarrowWarps, 2) narrow_items_kernel(StreamArgs a) {
   using G = typename Store<S>::G;
   __shared__ G red[kNarrowWarps * kNarrowRows];
   __shared__ int unit;
+  __shared__ int team_unit[kTeam ? kNarrowWarps : 1];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   // queue units [0, n_coop): the whole CTA per unit (queue[2] counts them)
   for (;;) {
@@ -1034,13 +1091,23 @@ __global__ void __launch_bounds__(32 * kNarrowWarps, 2) narrow_items_kernel(Stre
     if (u >= a.n_coop) break;
     narrow_unit_cta<S>(a, __ldg(a.item_ptr + u), __ldg(a.item_ptr + u + 1), lane, wid, red);
   }
-  // the rest: warp per unit (queue[0] counts them)
+  // the rest: a team of warps or a warp per unit (queue[0] counts them)
   for (;;) {
     int it = 0;
-    if (lane == 0) it = a.n_coop + atomicAdd(&a.queue[0], 1);
-    it = __shfl_sync(0xffffffffu, it, 0);
+    if constexpr (kTeam) {
+      if ((threadIdx.x & (32 * a.team - 1)) == 0) team_unit[wid] = a.n_coop + atomicAdd(&a.queue[0], 1);
+      bar_sync(1 + wid / a.team, 32 * a.team);
+      it = team_unit[wid & ~(a.team - 1)];
+    } else {
+      if (lane == 0) it = a.n_coop + atomicAdd(&a.queue[0], 1);
+      it = __shfl_sync(0xffffffffu, it, 0);
+    }
     if (it >= a.n_items) break;
-    narrow_unit_warp<S>(a, __ldg(a.item_ptr + it), __ldg(a.item_ptr + it + 1), lane);
+    const int cb = __ldg(a.item_ptr + it), ce = __ldg(a.item_ptr + it + 1);
+    if constexpr (kTeam)
+      narrow_unit_team<S>(a, cb, ce, lane, wid, a.team, red);
+    else
+      narrow_unit_warp<S>(a, cb, ce, lane);
   }
   // This CTA takes no more units; the last CTA returns the queue to zero.
   __syncthreads();

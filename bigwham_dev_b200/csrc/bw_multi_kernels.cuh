@@ -27,7 +27,6 @@
 namespace bw {
 
 constexpr int kMultiMax = 8;             // right-hand sides per pass
-constexpr int kMultiNarrowWarps = 8;     // unstaged kernel: warps per CTA, two CTAs per SM
 
 // Chunk's runs in the phase's run list (phase 2).
 struct RunRange {
@@ -405,31 +404,42 @@ __global__ void __launch_bounds__(threads_of<S>(), 1) stream_multi_kernel(MultiA
   }
 }
 
-// The unstaged kernel (narrow_items_kernel, warp per unit) with K columns.  A
-// warp first notes the source row of each of the chunk's columns in shared
-// memory (phase 1: the run of x starting at the chunk's vector offset).
+// The unstaged kernel (narrow_items_kernel: a team of warps per unit) with K
+// columns, one CTA of 16 warps per SM.  A warp first notes the source row of
+// each of the chunk's columns in shared memory (phase 1: the run of x starting
+// at the chunk's vector offset).
 template <typename S, int K>
-__global__ void __launch_bounds__(32 * kMultiNarrowWarps, 2) narrow_multi_kernel(MultiArgs m) {
+__global__ void __launch_bounds__(32 * kNarrowWarps, 1) narrow_multi_kernel(MultiArgs m) {
   using G = typename Store<S>::G;
   using V = typename std::conditional<sizeof(G) == 8, double2, float4>::type;
   constexpr int R = 16 / (int)sizeof(G);
   constexpr int kPer = 16 / (int)sizeof(G);
   constexpr int kAhead = sizeof(G) == 8 ? 4 : 6;
   const StreamArgs &a = m.s;
-  __shared__ uint32_t s_src[kMultiNarrowWarps][kMaxCols];
+  __shared__ uint32_t s_src[kNarrowWarps][kMaxCols];
+  __shared__ G red[kNarrowWarps * kNarrowRows];
+  __shared__ int team_unit[kNarrowWarps];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int team = a.team, tw = wid & (team - 1), w0 = wid - tw, bar = 1 + wid / team;
+  auto team_sync = [&]() {
+    if (team > 1)
+      bar_sync(bar, 32 * team);
+    else
+      __syncwarp();
+  };
   uint32_t *src = s_src[wid];
   const G *xk = static_cast<const G *>(m.xk), *tk = static_cast<const G *>(m.tk);
   const unsigned char *gdata = static_cast<const unsigned char *>(a.data);
   for (;;) {
-    int it = 0;
-    if (lane == 0) it = atomicAdd(&a.queue[0], 1);
-    it = __shfl_sync(0xffffffffu, it, 0);
+    if (tw == 0 && lane == 0) team_unit[w0] = atomicAdd(&a.queue[0], 1);
+    team_sync();
+    const int it = team_unit[w0];
+    team_sync();
     if (it >= a.n_items) break;
     const int cb = __ldg(a.item_ptr + it), ce = __ldg(a.item_ptr + it + 1);
     G acc[R][K];
     for (int i = cb; i < ce; i++) {
-      const NarrowChunk d = narrow_desc(a, i, lane == 0);
+      const NarrowChunk d = narrow_desc(a, i, tw == 0 && lane == 0);
       if (d.flags & kFirst) {
 #pragma unroll
         for (int r = 0; r < R; r++)
@@ -449,12 +459,12 @@ __global__ void __launch_bounds__(32 * kMultiNarrowWarps, 2) narrow_multi_kernel
         }
       }
       __syncwarp();
-      const int lpc = narrow_lpc(d.hpad, R), cpp = 32 / lpc;
+      const int lpc = narrow_lpc(d.hpad, R), cpp = (32 / lpc) * team;
       const int r0 = (lane % lpc) * R;
       if (r0 < d.hpad) {
         const G *db = reinterpret_cast<const G *>(gdata + d.data_off * Store<S>::kEsize) + r0;
 #pragma unroll 1
-        for (int c = lane / lpc; c < d.ncols; c += kAhead * cpp) {
+        for (int c = lane / lpc + (32 / lpc) * tw; c < d.ncols; c += kAhead * cpp) {
           V v[kAhead];
 #pragma unroll
           for (int q = 0; q < kAhead; q++) {
@@ -486,14 +496,33 @@ __global__ void __launch_bounds__(32 * kMultiNarrowWarps, 2) narrow_multi_kernel
           for (int r = 0; r < R; r++)
 #pragma unroll
             for (int j = 0; j < K; j++) acc[r][j] += __shfl_xor_sync(0xffffffffu, acc[r][j], o);
-        if (lane < lpc) {
+        if (team == 1) {
+          if (lane < lpc) {
 #pragma unroll
-          for (int r = 0; r < R; r++)
-            if (lane * R + r < d.rows) {
-              const long long dst = multi_row(a, d.out_off + lane * R + r);
+            for (int r = 0; r < R; r++)
+              if (lane * R + r < d.rows) {
+                const long long dst = multi_row(a, d.out_off + lane * R + r);
 #pragma unroll
-              for (int j = 0; j < K; j++) multi_store<G, K>(m, dst, j, acc[r][j]);
+                for (int j = 0; j < K; j++) multi_store<G, K>(m, dst, j, acc[r][j]);
+              }
+          }
+        } else {
+          // column by column: the warps' rows meet in red, summed in warp order
+#pragma unroll
+          for (int j = 0; j < K; j++) {
+            if (lane < lpc) {
+#pragma unroll
+              for (int r = 0; r < R; r++)
+                if (lane * R + r < d.hpad) red[wid * kNarrowRows + lane * R + r] = acc[r][j];
             }
+            team_sync();
+            for (int r = 32 * tw + lane; r < d.rows; r += 32 * team) {
+              G sum = red[w0 * kNarrowRows + r];
+              for (int w = 1; w < team; w++) sum += red[(w0 + w) * kNarrowRows + r];
+              multi_store<G, K>(m, multi_row(a, d.out_off + r), j, sum);
+            }
+            team_sync();
+          }
         }
       }
     }
