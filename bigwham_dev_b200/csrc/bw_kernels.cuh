@@ -52,6 +52,7 @@ struct StreamArgs {
   int n_items;
   int n_coop;                 // unstaged kernel: units [0, n_coop) run CTA-cooperatively
   int team;                   // unstaged kernel: warps per unit for the rest (1, 2, 4, 8 or 16)
+  int first;                  // unstaged kernel: the phase has no CTA-wide launch before this one
   int *queue;                 // [next item, CTAs done(, next CTA-cooperative unit)]: zero at launch, reset
                               // to zero by the last CTA
   const void *gsrc;           // vector values: gathered x (phase 1) or G2 (phase 2), compute type
@@ -125,6 +126,11 @@ __device__ __forceinline__ void pdl_launch_dependents() {
 }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// The gather wrote the vector with ordinary stores; the bulk copies read it
+// through the async proxy.
+__device__ __forceinline__ void fence_proxy_async_global() {
+  asm volatile("fence.proxy.async.global;" ::: "memory");
+}
 // Barrier `id` (1..15) over the `threads` threads that use it.
 __device__ __forceinline__ void bar_sync(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
@@ -370,6 +376,18 @@ __device__ __forceinline__ void load_desc(const Chunk *chunks, int idx, int end,
   }
 }
 
+// Bytes of a chunk's block data, and whether a descriptor is one the stages can
+// hold (a bad one is reported and read as an empty chunk).
+template <typename S> __device__ __forceinline__ unsigned long long chunk_bytes_of(const uint32_t (&w)[kChunkWords]) {
+  constexpr bool kTensor = Store<S>::kRows == 0;
+  const unsigned long long n = static_cast<unsigned long long>(static_cast<int>(w[2]));
+  return (kTensor ? (n + 7ull) & ~7ull : n) * static_cast<int>(w[3]) * Store<S>::kEsize;
+}
+template <typename S> __device__ __forceinline__ bool chunk_ok(const uint32_t (&w)[kChunkWords]) {
+  const int ncols = static_cast<int>(w[2]);
+  return ncols > 0 && ncols <= kMaxCols && chunk_bytes_of<S>(w) <= static_cast<unsigned long long>(kStageBytes);
+}
+
 template <typename S>
 __global__ void __launch_bounds__(threads_of<S>(), 1) stream_panels_kernel(StreamArgs a) {
   using G = typename Store<S>::G;
@@ -395,10 +413,6 @@ __global__ void __launch_bounds__(threads_of<S>(), 1) stream_panels_kernel(Strea
     fence_barrier_init();
   }
   __syncthreads();
-  // Every CTA is resident and holds its shared memory: a phase's unstaged
-  // launch (independent items, its own queue) may start filling the SMs this
-  // launch leaves free, and the SMs it frees as its CTAs run out of items.
-  pdl_launch_dependents();
 
   if (warp == 0) {
     // ------------------------------------------------------------------ producer
@@ -407,6 +421,32 @@ __global__ void __launch_bounds__(threads_of<S>(), 1) stream_panels_kernel(Strea
     const uint64_t stream_policy = l2_evict_first_policy();
     bool ok = true;
     int issued = 0;  // chunks staged so far by this CTA (stage = issued % kStages)
+    // Copy of a staged chunk's vector window (from the descriptor in its stage).
+    auto copy_window = [&](int s, int ncols, int g_off) {
+      const unsigned long long gs = reinterpret_cast<unsigned long long>(gvec) +
+                                    static_cast<unsigned long long>(g_off) * sizeof(G);
+      const unsigned long long glo = gs & ~15ull, ghi = (gs + ncols * sizeof(G) + 15ull) & ~15ull;
+      bulk_g2s(stage0 + s * L::kStageSize + L::kDataBytes, reinterpret_cast<const void *>(glo),
+               static_cast<uint32_t>(ghi - glo), &full[s]);
+    };
+    // The launch may start while the one before it (the gather that writes
+    // this phase's vector) still runs: block data, descriptors and the queue
+    // do not depend on it, so the first kStages chunks' data is requested
+    // before the wait and their vector windows after it.  Once every CTA has
+    // waited, the phase's unstaged launch (independent items, its own queue)
+    // or the next gather may start on the room this launch leaves.
+    bool ordered = false;
+    auto order = [&]() {
+      pdl_wait();
+      fence_proxy_async_global();
+      pdl_launch_dependents();
+      if (lane == 0)
+        for (int s = 0; s < issued; s++) {  // issued <= kStages here
+          const Chunk &d = *reinterpret_cast<const Chunk *>(stage0 + s * L::kStageSize + L::kDataBytes + L::kGBytes);
+          if (!(blockIdx.x == 0 && s == a.withhold)) copy_window(s, d.ncols, d.g_off);
+        }
+      ordered = true;
+    };
     ItemQueue iq;
     iq.init(a.item_ptr, a.n_items, a.queue, lane);
     // batches of up to 32 chunks of one item; lane k holds chunk k's
@@ -424,33 +464,32 @@ __global__ void __launch_bounds__(threads_of<S>(), 1) stream_panels_kernel(Strea
         for (int k = 0; k < nb; k++) {
           const int s = issued % kStages;
           const uint32_t use = static_cast<uint32_t>(issued / kStages);
+          uint32_t w[kChunkWords];
+#pragma unroll
+          for (int q = 0; q < kChunkWords; q++) w[q] = __shfl_sync(0xffffffffu, cur_d.w[q], k);
+          // before the first stage is used again, and before a chunk without a
+          // window (an empty one, or one refused below)
+          if (!ordered && (issued == kStages || !chunk_ok<S>(w))) order();
           if (!mbar_wait(&empty[s], (use & 1u) ^ 1u, a.spin_limit)) {
             if (lane == 0) set_error(a.err, kErrTimeoutEmpty);
             ok = false;
             break;
           }
-          uint32_t w[kChunkWords];
-#pragma unroll
-          for (int q = 0; q < kChunkWords; q++) w[q] = __shfl_sync(0xffffffffu, cur_d.w[q], k);
           // test hook: a withheld chunk is never staged, so its wait runs out
           const bool held = blockIdx.x == 0 && issued == a.withhold;
           if (lane == 0 && !held) {
             const long long data_off = static_cast<long long>((static_cast<unsigned long long>(w[1]) << 32) | w[0]);
             const int ncols = static_cast<int>(w[2]);
-            const int hpad = static_cast<int>(w[3]);
             const int g_off = static_cast<int>(w[7]);
             unsigned char *st = stage0 + s * L::kStageSize;
             uint4 *dd = reinterpret_cast<uint4 *>(st + L::kDataBytes + L::kGBytes);
 #pragma unroll
             for (int q = 0; q < kChunkWords / 4; q++)
               dd[q] = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
-            const unsigned long long cols = kTensor ? (static_cast<unsigned long long>(ncols) + 7ull) & ~7ull
-                                                    : static_cast<unsigned long long>(ncols);
-            const unsigned long long bytes = cols * hpad * es;
-            if (ncols > 0 && ncols <= kMaxCols && bytes <= static_cast<unsigned long long>(kStageBytes)) {
+            if (chunk_ok<S>(w)) {
               const unsigned long long src = reinterpret_cast<unsigned long long>(gdata) +
                                              static_cast<unsigned long long>(data_off) * es;
-              const unsigned long long lo = src & ~15ull, hi = (src + bytes + 15ull) & ~15ull;
+              const unsigned long long lo = src & ~15ull, hi = (src + chunk_bytes_of<S>(w) + 15ull) & ~15ull;
               const unsigned long long gs = reinterpret_cast<unsigned long long>(gvec) +
                                             static_cast<unsigned long long>(g_off) * sizeof(G);
               const unsigned long long glo = gs & ~15ull, ghi = (gs + ncols * sizeof(G) + 15ull) & ~15ull;
@@ -462,8 +501,7 @@ __global__ void __launch_bounds__(threads_of<S>(), 1) stream_panels_kernel(Strea
                               stream_policy);
               else
                 bulk_g2s(st, reinterpret_cast<const void *>(lo), static_cast<uint32_t>(hi - lo), &full[s]);
-              bulk_g2s(st + L::kDataBytes, reinterpret_cast<const void *>(glo), static_cast<uint32_t>(ghi - glo),
-                       &full[s]);
+              if (ordered) copy_window(s, ncols, g_off);
             } else {
               if (ncols > 0) set_error(a.err, kErrBadChunk);
               mbar_arrive(&full[s]);
@@ -480,6 +518,7 @@ __global__ void __launch_bounds__(threads_of<S>(), 1) stream_panels_kernel(Strea
       }
       cur_d = nxt_d;
     }
+    if (!ordered) order();
     if (ok) {
       // end of work: a descriptor with kEnd alone, no data
       const int s = issued % kStages;
@@ -1082,6 +1121,10 @@ __global__ void __launch_bounds__(32 * kNarrowWarps, 2) narrow_items_kernel(Stre
   __shared__ int unit;
   __shared__ int team_unit[kTeam ? kNarrowWarps : 1];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  // As a phase's only launch it may start while the gather before it runs; as
+  // the second one it only starts once the CTA-wide launch has waited for that.
+  if (a.first) pdl_wait();
+  pdl_launch_dependents();
   // queue units [0, n_coop): the whole CTA per unit (queue[2] counts them)
   for (;;) {
     if (threadIdx.x == 0) unit = atomicAdd(&a.queue[2], 1);
@@ -1136,8 +1179,9 @@ __device__ __forceinline__ uint32_t pack_hilo(float v) {
 
 // G2[dst + c] = scale * src[src_off + c] for every run (src: gathered x or t):
 // the phase-2 vector values laid out chunk by chunk.  Runs are short (10 to
-// 60 values), so a warp takes kG2Runs = 32 of them at once and deals their
-// values to its lanes densely: lane k loads run k's descriptor and a warp
+// 60 values), so a warp takes up to kG2Runs = 32 of them at once (fewer where
+// that leaves the chip short of warps, g2_runs_per_warp) and deals their values
+// to its lanes densely: lane k loads run k's descriptor and a warp
 // scan gives each run its first position in the warp's value list.  A round
 // covers 32 consecutive positions [w0, w0 + 32): the run holding w0 is the
 // last one starting at or before it (one ballot), every later run starting
@@ -1151,14 +1195,27 @@ __device__ __forceinline__ uint32_t pack_hilo(float v) {
 constexpr int kG2Runs = 32;
 constexpr int kG2Unroll = 4;  // rounds in flight per lane
 
+// Runs per warp: a warp's rounds follow one another at the latency of a load,
+// 9 to 14 of them for 32 runs, so a list that does not fill the resident warps
+// (64 per SM) is dealt thinner.
+inline int g2_runs_per_warp(long long n_runs, int sms) {
+  int r = kG2Runs;
+  while (r > 2 && n_runs <= 64LL * sms * (r / 2)) r >>= 1;
+  return r;
+}
+
 template <typename G, bool kPacked>
-__global__ void gather_g2_kernel(const GatherSeg *__restrict__ runs, int n_runs, const G *__restrict__ xp,
+__global__ void gather_g2_kernel(const GatherSeg *__restrict__ runs, int n_runs, int per_warp,
+                                 const G *__restrict__ xp,
                                  const G *__restrict__ t, void *__restrict__ g2) {
   const int lane = threadIdx.x & 31;
-  const int r0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * kG2Runs;
-  if (r0 >= n_runs) return;  // warp-uniform
+  const int r0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * per_warp;
+  if (r0 >= n_runs) {  // warp-uniform
+    pdl_wait();  // the launch completes after phase 1 in any case
+    return;
+  }
   GatherSeg mine{};          // cols = 0 past the end
-  if (r0 + lane < n_runs) mine = runs[r0 + lane];
+  if (lane < per_warp && r0 + lane < n_runs) mine = runs[r0 + lane];
   const int cols = static_cast<int>(mine.cols_src & 0x7fffffffu);
   int incl = cols;  // inclusive scan of the run lengths over the lanes
 #pragma unroll
@@ -1169,6 +1226,8 @@ __global__ void gather_g2_kernel(const GatherSeg *__restrict__ runs, int n_runs,
   const int start = incl - cols;
   const int total = __shfl_sync(0xffffffffu, incl, 31);
   const unsigned below = (2u << lane) - 1u;  // bits 0..lane
+  pdl_wait();  // phase 1 is complete (its runs are read above, x and t below)
+  pdl_launch_dependents();
   for (int base = 0; base < total; base += 32 * kG2Unroll) {
     G v[kG2Unroll];
     int dst[kG2Unroll];
@@ -1211,6 +1270,7 @@ __global__ void gather_g2_kernel(const GatherSeg *__restrict__ runs, int n_runs,
 template <typename G>
 __global__ void gather_x_kernel(const double *__restrict__ x, G *__restrict__ xp, uint32_t *__restrict__ xpk,
                                 const int32_t *__restrict__ perm, int dof, int n) {
+  pdl_launch_dependents();  // phase 1 may start its block data copies
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int src = perm ? dof * perm[i / dof] + (i % dof) : i;

@@ -215,6 +215,10 @@ __global__ void __launch_bounds__(kMmThreads, 1) mm_stream_kernel(MmArgs a) {
     int bb = iq.cb;
     uint32_t dw[kMmChunkWords];
     load(bb, iq.ce, dw);
+    // the launch may have started before the one that writes X or T8 is done
+    pdl_wait();
+    fence_proxy_async_global();
+    pdl_launch_dependents();
     while (iq.valid() && ok) {
       const int be = min(bb + 32, iq.ce);
       const bool same = be < iq.ce;
@@ -521,6 +525,7 @@ __global__ void __launch_bounds__(256) gather_xt_kernel(const double *__restrict
                                                         uint16_t *__restrict__ xt, const int32_t *__restrict__ perm,
                                                         int dof, int n, int n_pad) {
   __shared__ float tile[64][kMmRhs + 1];
+  pdl_launch_dependents();
   const int i0 = blockIdx.x * 64;
   // a thread keeps one row and takes every fourth column: one permutation
   // lookup, then kMmRhs / 4 loads in flight (16.8 us at 27,648 rows with the

@@ -157,7 +157,6 @@ __global__ void __launch_bounds__(threads_of<S>(), 1) stream_multi_kernel(MultiA
     fence_barrier_init();
   }
   __syncthreads();
-  pdl_launch_dependents();
 
   if (warp == 0) {
     // ------------------------------------------------------------------ producer
@@ -181,6 +180,10 @@ __global__ void __launch_bounds__(threads_of<S>(), 1) stream_multi_kernel(MultiA
     RunRange cur_r = load_range(bb + lane, iq.ce);
     int first = __shfl_sync(0xffffffffu, cur_r.first, 0), count = __shfl_sync(0xffffffffu, cur_r.count, 0);
     GatherSeg run = load_run(first, count);
+    // the launch may have started before the one that writes x or t is done
+    pdl_wait();
+    fence_proxy_async_global();
+    pdl_launch_dependents();
     while (iq.valid() && ok) {
       const int be = min(bb + 32, iq.ce);
       const bool same = be < iq.ce;
@@ -430,6 +433,8 @@ __global__ void __launch_bounds__(32 * kNarrowWarps, 1) narrow_multi_kernel(Mult
   uint32_t *src = s_src[wid];
   const G *xk = static_cast<const G *>(m.xk), *tk = static_cast<const G *>(m.tk);
   const unsigned char *gdata = static_cast<const unsigned char *>(a.data);
+  if (a.first) pdl_wait();  // as in narrow_items_kernel
+  pdl_launch_dependents();
   for (;;) {
     if (tw == 0 && lane == 0) team_unit[w0] = atomicAdd(&a.queue[0], 1);
     team_sync();
@@ -545,6 +550,7 @@ template <typename G, int K>
 __global__ void __launch_bounds__(256) gather_xk_kernel(const double *__restrict__ x, long long ldx, int nrhs,
                                                         G *__restrict__ xk, const int32_t *__restrict__ perm, int dof,
                                                         int n) {
+  pdl_launch_dependents();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const long long src = perm ? static_cast<long long>(dof) * perm[i / dof] + (i % dof) : i;
