@@ -17,8 +17,8 @@
 // number of barriers (ten, at any rank: two CTA reductions per earlier rank
 // block took most of the time before), and the blocks come from a queue,
 // longest first, so that the largest does not start last.
-// A 64 x 64 crack's 1,584 blocks with the full-rank blocks: 28.0 -> 19.4 ms
-// through DeviceKernels.
+// A 64 x 64 crack's 1,584 blocks: 18.5 ms at first, 9.5 ms with this pass and
+// the queue, about 4 ms with a launch per size (kAcaSide).
 // Every stop decision is taken from values in shared memory that all threads
 // read, so all threads leave the loop together.  Factor storage per block is
 // capacity-bounded (cap blocks of rank); a block that needs more reports
@@ -26,12 +26,18 @@
 #pragma once
 
 #include "bw_aca.h"
+#include "bw_kernels.cuh"
 #include "bw_r0.h"
 
 namespace bw {
 
-constexpr int kAcaThreads = 128;
-constexpr int kAcaWarps = kAcaThreads / 32;
+// Threads per block of points: a warp for blocks of up to kAcaSide[0] points a
+// side, whose bands one warp covers in one or two rounds, 128 up to kAcaSide[1],
+// 512 above.  With 128 threads for all, three of the four warps of a 32-point
+// block waited at barriers and held registers, and each of a 64 x 64 crack's 24
+// blocks of 512 points took 9 ms, as long as the whole launch.
+constexpr int kAcaSide[2] = {48, 128};
+constexpr int kAcaResident = 512;  // threads per SM that the registers are limited for
 
 struct AcaBlock {
   long long a_off, b_off;  // factor storage (doubles): A n0 3 x cap 3, B cap 3 x n1 3, column-major
@@ -40,9 +46,16 @@ struct AcaBlock {
   int cap, pad;            // rank capacity in blocks
 };
 
+template <int NT> __device__ __forceinline__ void aca_sync() {
+  if constexpr (NT == 32)
+    __syncwarp();
+  else
+    __syncthreads();
+}
+
 // CTA argmax of (value, index) pairs: largest value, smallest index on ties;
 // index -1 when no thread had a candidate.
-__device__ __forceinline__ void aca_argmax(double v, int idx, double *sv, int *si, int &bi) {
+template <int NT> __device__ __forceinline__ void aca_argmax(double v, int idx, double *sv, int *si, int &bi) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   auto better = [](double v2, int i2, double v1, int i1) {
     return i2 >= 0 && (i1 < 0 || v2 > v1 || (v2 == v1 && i2 < i1));
@@ -60,15 +73,15 @@ __device__ __forceinline__ void aca_argmax(double v, int idx, double *sv, int *s
     sv[warp] = v;
     si[warp] = idx;
   }
-  __syncthreads();
+  aca_sync<NT>();
   bi = si[0];
   double best = sv[0];
-  for (int w = 1; w < kAcaWarps; w++)
+  for (int w = 1; w < (NT / 32); w++)
     if (better(sv[w], si[w], best, bi)) {
       best = sv[w];
       bi = si[w];
     }
-  __syncthreads();
+  aca_sync<NT>();
 }
 
 // K -= A B over `rank` scalar columns: A's three rows of one point, B's three
@@ -90,15 +103,16 @@ __device__ __forceinline__ void aca_subtract(const double *A, long long lda, con
 
 constexpr int kAcaPass = 32;  // earlier rank blocks whose Frobenius terms one pass takes (a lane each)
 
-struct AcaFrob {
-  double m1[kAcaPass][9];             // A_r^T A_k
-  double m2[kAcaWarps][9][kAcaPass];  // per warp: part of (B_k B_r^T)^T
+template <int NT> struct AcaFrob {
+  double m1[kAcaPass][9];           // A_r^T A_k
+  double m2[NT / 32][9][kAcaPass];  // per warp: part of (B_k B_r^T)^T
 };
 
 // Frobenius products <A_r B_r, A_k B_k>_F for r = 0 .. k: their sum over r < k
 // in `cross` and the term r = k in `self` (all threads).
+template <int NT>
 __device__ __forceinline__ void aca_frobenius(const double *A, long long lda, const double *B, long long ldb, int k,
-                                              long long cols, AcaFrob &f, double *s_out, double &cross,
+                                              long long cols, AcaFrob<NT> &f, double *s_out, double &cross,
                                               double &self) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   cross = 0.0;
@@ -107,9 +121,10 @@ __device__ __forceinline__ void aca_frobenius(const double *A, long long lda, co
   for (int r0 = 0; r0 <= k; r0 += kAcaPass) {
     const int nr = min(kAcaPass, k + 1 - r0);
     // warp: one r at a time, lanes along the rows
-    for (int q = warp; q < nr; q += kAcaWarps) {
+    for (int q = warp; q < nr; q += (NT / 32)) {
       const double *Ar = A + 3LL * (r0 + q) * lda;
       double m[9] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+#pragma unroll 2
       for (long long i = lane; i < lda; i += 32) {
         const double a0 = Ar[i], a1 = Ar[lda + i], a2 = Ar[2 * lda + i];
 #pragma unroll
@@ -132,8 +147,8 @@ __device__ __forceinline__ void aca_frobenius(const double *A, long long lda, co
     double m[9] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     if (lane < nr) {
       const double *Br = B + 3LL * (r0 + lane), *Bk = B + 3LL * k;
-#pragma unroll 2
-      for (long long j = warp; j < cols; j += kAcaWarps) {
+#pragma unroll 4
+      for (long long j = warp; j < cols; j += (NT / 32)) {
         const double *c = Br + j * ldb, *d = Bk + j * ldb;
         const double a0 = c[0], a1 = c[1], a2 = c[2];
 #pragma unroll
@@ -146,14 +161,14 @@ __device__ __forceinline__ void aca_frobenius(const double *A, long long lda, co
     }
 #pragma unroll
     for (int e = 0; e < 9; e++) f.m2[warp][e][lane] = m[e];
-    __syncthreads();
+    aca_sync<NT>();
     if (warp == 0) {
       double v = 0.0;
       if (lane < nr)
 #pragma unroll
         for (int e = 0; e < 9; e++) {
           double m2 = f.m2[0][e][lane];
-          for (int w = 1; w < kAcaWarps; w++) m2 += f.m2[w][e][lane];
+          for (int w = 1; w < (NT / 32); w++) m2 += f.m2[w][e][lane];
           v += f.m1[lane][e] * m2;
         }
       const bool last = r0 + lane == k;
@@ -166,29 +181,29 @@ __device__ __forceinline__ void aca_frobenius(const double *A, long long lda, co
         s_out[1] = own;
       }
     }
-    __syncthreads();
+    aca_sync<NT>();
     cross += s_out[0];
     self = s_out[1];  // the last pass holds r = k
   }
 }
 
-__global__ void __launch_bounds__(kAcaThreads) r0_aca_kernel(const double *__restrict__ records,
-                                                             const int *__restrict__ perm,
-                                                             const AcaBlock *__restrict__ blocks, int n_blocks,
-                                                             double G, double nu, double eps, double *factors_a,
-                                                             double *factors_b, double *scratch,
-                                                             long long slot_doubles, const int *order, int *queue,
-                                                             int *rank_out, double *err_out) {
-  __shared__ double s_val[kAcaWarps];
-  __shared__ int s_idx[kAcaWarps];
-  __shared__ AcaFrob s_frob;
+template <int NT>
+__global__ void __launch_bounds__(NT, kAcaResident / NT)
+    r0_aca_kernel(const double *__restrict__ records, const int *__restrict__ perm,
+                  const AcaBlock *__restrict__ blocks, int n_blocks, double G, double nu, double eps,
+                  double *factors_a, double *factors_b, double *scratch, long long slot_doubles, const int *order,
+                  int *queue, int *rank_out, double *err_out) {
+  __shared__ double s_val[NT / 32];
+  __shared__ int s_idx[NT / 32];
+  __shared__ AcaFrob<NT> s_frob;
   __shared__ double s_gamma[9], s_sum[2];
   __shared__ int s_ctl[2];  // [0] continue, [1] the CTA's next block
   const int t = threadIdx.x;
+  pdl_launch_dependents();  // the other size's launch, independent of this one, may run beside it
   double *row = scratch + (long long)blockIdx.x * slot_doubles;  // 3 x n1 3 (ld 3)
   for (;;) {
     if (t == 0) s_ctl[1] = atomicAdd(queue, 1);
-    __syncthreads();
+    aca_sync<NT>();
     const int place = s_ctl[1];
     if (place >= n_blocks) break;
     const int bk = order[place];
@@ -199,9 +214,9 @@ __global__ void __launch_bounds__(kAcaThreads) r0_aca_kernel(const double *__res
     double *Bf = factors_b + B_.b_off;
     int *used0 = reinterpret_cast<int *>(row + 9LL * n1);
     int *used1 = used0 + n0;
-    for (int i = t; i < n0; i += kAcaThreads) used0[i] = 0;
-    for (int j = t; j < n1; j += kAcaThreads) used1[j] = 0;
-    __syncthreads();
+    for (int i = t; i < n0; i += NT) used0[i] = 0;
+    for (int j = t; j < n1; j += NT) used1[j] = 0;
+    aca_sync<NT>();
     auto entry = [&](int i, int j, double K[3][3]) {
       const double *src = records + r0::kFrameDoubles * perm[B_.j0 + j];
       const double *rec = records + r0::kFrameDoubles * perm[B_.i0 + i];
@@ -216,7 +231,7 @@ __global__ void __launch_bounds__(kAcaThreads) r0_aca_kernel(const double *__res
         break;
       }
       // residual row band of row block i0
-      for (int j = t; j < n1; j += kAcaThreads) {
+      for (int j = t; j < n1; j += NT) {
         double K[3][3];
         entry(i0, j, K);
         aca_subtract(A + 3LL * i0, lda, Bf + 3LL * j * ldb, ldb, 3 * rank, K);
@@ -225,11 +240,11 @@ __global__ void __launch_bounds__(kAcaThreads) r0_aca_kernel(const double *__res
 #pragma unroll
           for (int a = 0; a < 3; a++) row[(3LL * j + b) * 3 + a] = K[a][b];
       }
-      __syncthreads();
+      aca_sync<NT>();
       // pivot column block
       double best = 0.0;
       int bi = -1;
-      for (int j = t; j < n1; j += kAcaThreads) {
+      for (int j = t; j < n1; j += NT) {
         if (used1[j]) continue;
         const double sv = aca::smallest_singular_value(row + 9LL * j);
         if (sv > best) {  // ascending j per thread: the first maximum stays
@@ -238,17 +253,17 @@ __global__ void __launch_bounds__(kAcaThreads) r0_aca_kernel(const double *__res
         }
       }
       int i1;
-      aca_argmax(best, bi, s_val, s_idx, i1);
+      aca_argmax<NT>(best, bi, s_val, s_idx, i1);
       if (i1 < 0) break;  // uniform: every thread read the same i1
       if (t == 0) {
         used0[i0] = 1;
         used1[i1] = 1;
         s_ctl[0] = aca::invert3(row + 9LL * i1, s_gamma) ? 1 : 0;
       }
-      __syncthreads();
+      aca_sync<NT>();
       if (!s_ctl[0]) break;
       // A_k: residual column band of column block i1
-      for (int i = t; i < n0; i += kAcaThreads) {
+      for (int i = t; i < n0; i += NT) {
         double K[3][3];
         entry(i, i1, K);
         aca_subtract(A + 3LL * i, lda, Bf + 3LL * i1 * ldb, ldb, 3 * rank, K);
@@ -258,21 +273,21 @@ __global__ void __launch_bounds__(kAcaThreads) r0_aca_kernel(const double *__res
           for (int a = 0; a < 3; a++) A[(3LL * rank + b) * lda + 3LL * i + a] = K[a][b];
       }
       // B_k = Gamma R
-      for (int j = t; j < 3 * n1; j += kAcaThreads)
+      for (int j = t; j < 3 * n1; j += NT)
         for (int a = 0; a < 3; a++) {
           double v = 0.0;
           for (int c = 0; c < 3; c++) v += s_gamma[c * 3 + a] * row[3LL * j + c];
           Bf[(long long)j * ldb + 3LL * rank + a] = v;
         }
-      __syncthreads();
+      aca_sync<NT>();
       // |A_k B_k|_F^2 and cross terms with the earlier rank blocks
       double ab, cross;
-      aca_frobenius(A, lda, Bf, ldb, rank, 3LL * n1, s_frob, s_sum, cross, ab);
+      aca_frobenius<NT>(A, lda, Bf, ldb, rank, 3LL * n1, s_frob, s_sum, cross, ab);
       s_norm += 2.0 * cross + ab;
       // next row block from A_k
       best = 0.0;
       bi = -1;
-      for (int i = t; i < n0; i += kAcaThreads) {
+      for (int i = t; i < n0; i += NT) {
         if (used0[i]) continue;
         double blk[9];
         for (int b = 0; b < 3; b++)
@@ -284,7 +299,7 @@ __global__ void __launch_bounds__(kAcaThreads) r0_aca_kernel(const double *__res
         }
       }
       int next;
-      aca_argmax(best, bi, s_val, s_idx, next);
+      aca_argmax<NT>(best, bi, s_val, s_idx, next);
       rank++;
       if (next < 0 || rank == max_rank) break;
       if (fabs(ab) <= eps * eps * fabs(s_norm)) {
@@ -297,8 +312,9 @@ __global__ void __launch_bounds__(kAcaThreads) r0_aca_kernel(const double *__res
       rank_out[bk] = status == 2 ? -1 : rank;
       err_out[bk] = err;
     }
-    __syncthreads();
+    aca_sync<NT>();
   }
+  pdl_wait();  // completes after the launch before it
 }
 
 }  // namespace bw

@@ -27,7 +27,7 @@ struct AsmTile {
   int block, ti, tj, pad;  // block, first row / column point inside it
 };
 
-__global__ void __launch_bounds__(kAsmTile *kAsmTile) r0_fr_assemble_kernel(
+__global__ void __launch_bounds__(kAsmTile *kAsmTile, 2) r0_fr_assemble_kernel(
     const double *__restrict__ records, const int *__restrict__ perm, const AsmBlock *__restrict__ blocks,
     const AsmTile *__restrict__ tiles, long long n_tiles, double G, double nu, double *__restrict__ out) {
   for (long long t = blockIdx.x; t < n_tiles; t += gridDim.x) {

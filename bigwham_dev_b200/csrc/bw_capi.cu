@@ -2094,43 +2094,61 @@ int bw_r0_aca(int device, int64_t n_elems, const double *records, double G, doub
     std::stable_sort(order.begin(), order.end(), [&](int32_t p, int32_t q) {
       return blocks[p].n0 + blocks[p].n1 > blocks[q].n0 + blocks[q].n1;
     });
-    order.push_back(0);  // the kernel's queue counter
+    // three launches by size, each with its part of the order, its queue
+    // counter (behind the order) and its rows of scratch
+    auto size_class = [&](int32_t k) {
+      const int side = std::max(blocks[k].n0, blocks[k].n1);
+      return side > bw::kAcaSide[1] ? 0 : side > bw::kAcaSide[0] ? 1 : 2;
+    };
+    std::stable_sort(order.begin(), order.end(), [&](int32_t p, int32_t q) { return size_class(p) < size_class(q); });
+    const int threads[3] = {512, 128, 32};
+    int64_t first[4] = {0, 0, 0, n_lr}, slots[3], scratch_at[4] = {0};
+    int ctas[3];
+    for (int c = 0; c < 3; c++) {
+      if (c > 0)
+        first[c] = std::partition_point(order.begin(), order.end(), [&](int32_t k) { return size_class(k) < c; }) -
+                   order.begin();
+      slots[c] = c == 0 ? slot : 11 * bw::kAcaSide[2 - c] + 2;
+    }
+    for (int c = 0; c < 3; c++) {
+      ctas[c] = (int)std::min<int64_t>(first[c + 1] - first[c], 148 * (bw::kAcaResident / threads[c]));
+      scratch_at[c + 1] = scratch_at[c] + slots[c] * ctas[c];
+    }
+    order.insert(order.end(), 3, 0);
     BW_CUDA(cudaSetDevice(device));
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const int grid = (int)std::min<int64_t>(n_lr, 148 * 4);
-    void *d_rec = nullptr, *d_perm = nullptr, *d_blk = nullptr, *d_scr = nullptr, *d_rank = nullptr, *d_err = nullptr,
-         *d_ord = nullptr;
-    auto release = [&] {
-      for (void *q : {d_rec, d_perm, d_blk, d_scr, d_rank, d_err, d_ord}) cudaFree(q);
-    };
+    // one device allocation for the call's tables, scratch and results
+    const int64_t parts[7] = {8 * (int64_t)bw::r0::kFrameDoubles * n_elems, 4 * (int64_t)p32.size(),
+                              (int64_t)(sizeof(bw::AcaBlock) * blocks.size()), 4 * (int64_t)order.size(),
+                              8 * scratch_at[3], 4 * n_lr, 8 * n_lr};
+    int64_t at[8] = {0};
+    for (int k = 0; k < 7; k++) at[k + 1] = at[k] + align256(parts[k]);
+    DevTemp arena((size_t)at[7]);
+    unsigned char *d = arena.as<unsigned char>();
     try {
-      const size_t rb = sizeof(double) * bw::r0::kFrameDoubles * (size_t)n_elems;
-      BW_CUDA(cudaMalloc(&d_rec, rb));
-      BW_CUDA(cudaMalloc(&d_perm, 4 * p32.size()));
-      BW_CUDA(cudaMalloc(&d_blk, sizeof(bw::AcaBlock) * blocks.size()));
-      BW_CUDA(cudaMalloc(&d_scr, sizeof(double) * (size_t)slot * grid));
-      BW_CUDA(cudaMalloc(&d_rank, 4 * (size_t)n_lr));
-      BW_CUDA(cudaMalloc(&d_err, 8 * (size_t)n_lr));
-      BW_CUDA(cudaMalloc(&d_ord, 4 * order.size()));
-      BW_CUDA(cudaMemcpyAsync(d_ord, order.data(), 4 * order.size(), cudaMemcpyHostToDevice, st));
-      BW_CUDA(cudaMemcpyAsync(d_rec, records, rb, cudaMemcpyHostToDevice, st));
-      BW_CUDA(cudaMemcpyAsync(d_perm, p32.data(), 4 * p32.size(), cudaMemcpyHostToDevice, st));
-      BW_CUDA(cudaMemcpyAsync(d_blk, blocks.data(), sizeof(bw::AcaBlock) * blocks.size(), cudaMemcpyHostToDevice, st));
-      bw::r0_aca_kernel<<<grid, bw::kAcaThreads, 0, st>>>(
-          static_cast<const double *>(d_rec), static_cast<const int *>(d_perm),
-          static_cast<const bw::AcaBlock *>(d_blk), (int)n_lr, G, nu, eps, factors_a, factors_b,
-          static_cast<double *>(d_scr), slot, static_cast<const int *>(d_ord), static_cast<int *>(d_ord) + n_lr,
-          static_cast<int *>(d_rank), static_cast<double *>(d_err));
-      BW_CUDA(cudaGetLastError());
+      const void *up[4] = {records, p32.data(), blocks.data(), order.data()};
+      for (int k = 0; k < 4; k++)
+        BW_CUDA(cudaMemcpyAsync(d + at[k], up[k], (size_t)parts[k], cudaMemcpyHostToDevice, st));
+      int *d_order = reinterpret_cast<int *>(d + at[3]), *d_rank = reinterpret_cast<int *>(d + at[5]);
+      double *d_scr = reinterpret_cast<double *>(d + at[4]), *d_err = reinterpret_cast<double *>(d + at[6]);
+      bool early = false;  // the launches are independent: a later one may run beside the one before it
+      for (int c = 0; c < 3; c++) {
+        const int64_t n = first[c + 1] - first[c];
+        if (n == 0) continue;
+        launch(c == 0 ? bw::r0_aca_kernel<512> : c == 1 ? bw::r0_aca_kernel<128> : bw::r0_aca_kernel<32>, ctas[c],
+               threads[c], 0, st, early, reinterpret_cast<const double *>(d + at[0]),
+               reinterpret_cast<const int *>(d + at[1]), reinterpret_cast<const bw::AcaBlock *>(d + at[2]), (int)n, G,
+               nu, eps, factors_a, factors_b, d_scr + scratch_at[c], (long long)slots[c], d_order + first[c],
+               d_order + n_lr + c, d_rank, d_err);
+        early = true;
+      }
       BW_CUDA(cudaMemcpyAsync(rank_out, d_rank, 4 * (size_t)n_lr, cudaMemcpyDeviceToHost, st));
       BW_CUDA(cudaMemcpyAsync(err_out, d_err, 8 * (size_t)n_lr, cudaMemcpyDeviceToHost, st));
       BW_CUDA(cudaStreamSynchronize(st));
     } catch (...) {
       cudaStreamSynchronize(st);
-      release();
       throw;
     }
-    release();
     for (int64_t k = 0; k < n_lr; k++)
       if (rank_out[k] > 0) rank_out[k] *= 3;  // scalar rank (LRB_pattern flag); -1: capacity too small
     return BW_OK;

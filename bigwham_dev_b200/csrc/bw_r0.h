@@ -219,6 +219,19 @@ BW_HD Derivs derivs(double x, double y, double z, double a, double b) {
   return z == 0.0 ? derivs_inplane(x, y, a, b) : derivs_offplane(x, y, z, a, b);
 }
 
+// derivs with the off-plane case as a call: entries between elements of one
+// plane, all of them on a planar crack, then do not hold its registers.
+#ifdef __CUDACC__
+static __host__ __device__ __noinline__ void derivs_offplane_call(double x, double y, double z, double a, double b,
+                                                                  Derivs *d) {
+  *d = derivs_offplane(x, y, z, a, b);
+}
+#else
+inline void derivs_offplane_call(double x, double y, double z, double a, double b, Derivs *d) {
+  *d = derivs_offplane(x, y, z, a, b);
+}
+#endif
+
 // Stresses in the element's local frame: s[dd][c], dd = DD x, y, z and
 // c = xx, yy, zz, xy, xz, yz (the reference's StressesKernelR0 layout), from
 // the derivatives at (x, y, z); stress() evaluates them first.
@@ -289,7 +302,13 @@ BW_HD void influence_h(const double *cp_s, const double *rot_s, double a_s, doub
     nl[r] = rot_s[3 * r] * n_r[0] + rot_s[3 * r + 1] * n_r[1] + rot_s[3 * r + 2] * n_r[2];
   }
   double s[3][6];
-  stress(dl[0], dl[1], dl[2], a_s, b_s, G, nu, s);
+  if (dl[2] == 0.0) {
+    stress_from(derivs_inplane(dl[0], dl[1], a_s, b_s), 0.0, G, nu, s);
+  } else {
+    Derivs D;
+    derivs_offplane_call(dl[0], dl[1], dl[2], a_s, b_s, &D);
+    stress_from(D, dl[2], G, nu, s);
+  }
   for (int i = 0; i < 3; i++) {
     // traction on nl in the source frame (symmetric tensor xx yy zz xy xz yz)
     const double t0 = s[i][0] * nl[0] + s[i][3] * nl[1] + s[i][4] * nl[2];
