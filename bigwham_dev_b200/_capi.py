@@ -69,6 +69,7 @@ _SIGS = {
                             _P, _I64, _P, _I64, _P, _P, _P]),
     "bw_s0_fields": (C.c_int, [C.c_int, _I64, _P, _P, C.c_double, C.c_double, _I64, _P, _P, _P, _P]),
     "bw_r0_fields": (C.c_int, [C.c_int, _I64, _P, _P, C.c_double, C.c_double, _I64, _P, _P, _P, _P]),
+    "bw_arnoldi_step": (C.c_int, [C.c_int, _I64, C.c_int, C.c_int, _P, _P, _P, _P, _P, _P, _I64, C.c_double, _P]),
     "bw_destroy": (C.c_int, [_P]),
     "bw_version": (C.c_char_p, []),
 }

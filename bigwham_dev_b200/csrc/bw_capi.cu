@@ -17,6 +17,7 @@
 #include "bw_mm_kernels.cuh"
 #include "bw_multi_kernels.cuh"
 #include "bw_aca_kernels.cuh"
+#include "bw_arnoldi_kernels.cuh"
 #include "bw_assemble_kernels.cuh"
 #include "bw_devlayout_kernels.cuh"
 #include "bw_fields_kernels.cuh"
@@ -2154,6 +2155,29 @@ int bw_r0_aca(int device, int64_t n_elems, const double *records, double G, doub
     }
     for (int64_t k = 0; k < n_lr; k++)
       if (rank_out[k] > 0) rank_out[k] *= 3;  // scalar rank (LRB_pattern flag); -1: capacity too small
+    return BW_OK;
+  });
+}
+
+int bw_arnoldi_step(int device, int64_t n, int j, int m, double *V, double *H, double *w, const double *minv,
+                    double *z, double *work, int64_t work_len, double breakdown, void *stream) {
+  return device_guarded([&] {
+    if (n < 1 || m < 1 || j < 0 || j >= m || !V || !H || !w || !work || !minv != !z)
+      throw std::invalid_argument("bw_arnoldi_step: null or out-of-range argument");
+    if (m > bw::kArnoldiMaxSteps) throw std::invalid_argument("bw_arnoldi_step: m too large");
+    if (work_len < 3 * (int64_t)(m + 2)) throw std::invalid_argument("bw_arnoldi_step: work too small");
+    BW_CUDA(cudaSetDevice(device));
+    int sms = 0;
+    BW_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    const int grid = (int)std::max<int64_t>(
+        1, std::min<int64_t>({(int64_t)sms, (n + 63) / 64, work_len / (3 * (int64_t)(m + 2))}));
+    bw::ArnoldiArgs a{V, H, w, minv, z, work, (long long)n, j, m, breakdown};
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const size_t smem = sizeof(double) * (size_t)(m + 2);
+    launch(bw::arnoldi_kernel<0>, grid, bw::kArnoldiThreads, smem, st, false, a);
+    launch(bw::arnoldi_kernel<1>, grid, bw::kArnoldiThreads, smem, st, true, a);
+    launch(bw::arnoldi_kernel<2>, grid, bw::kArnoldiThreads, smem, st, true, a);
+    launch(bw::arnoldi_kernel<3>, grid, bw::kArnoldiThreads, smem, st, true, a);
     return BW_OK;
   });
 }

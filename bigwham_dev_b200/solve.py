@@ -28,6 +28,8 @@ from dataclasses import dataclass, field
 
 import numpy as np
 
+from . import _capi as A
+
 
 @dataclass
 class SolveInfo:
@@ -83,9 +85,32 @@ class Gmres:
         self.w = torch.zeros(self.n, dtype=dt, device=device)
         self.use_graph = use_graph
         self.graph = None
+        # CUDA: the step after the operator runs in the library's own kernels
+        # (bw_arnoldi_step, up to 4,096 steps a cycle)
+        self._work = None
+        if self.V.is_cuda and self.m <= 4096:
+            self._work = torch.empty(3 * 160 * (self.m + 2), dtype=dt, device=self.V.device)
+
+    def _device_cycle(self):
+        """_cycle with each step's Gram-Schmidt in four launches."""
+        V, z, w = self.V, self.z, self.w
+        dev = V.device.index
+        step, stream = A.lib().bw_arnoldi_step, self.torch.cuda.current_stream(dev).cuda_stream
+        d = self.minv  # a plain diagonal multiplies in the step's last launch
+        fused = (isinstance(d, self.torch.Tensor) and d.dtype == V.dtype and d.device == V.device
+                 and d.shape == (self.n,) and d.is_contiguous())
+        minv, zp = (d.data_ptr(), z.data_ptr()) if fused else (0, 0)
+        for j in range(self.m):
+            if j == 0 or not fused:
+                self._precondition(V[j], z)
+            self.op(z, w)
+            A.check(step(dev, self.n, j, self.m, V.data_ptr(), self.H.data_ptr(), w.data_ptr(), minv, zp,
+                         self._work.data_ptr(), self._work.numel(), _BREAKDOWN, stream), None)
 
     def _cycle(self):
         """m Arnoldi steps from V[0]; fills V and H (FP64)."""
+        if self._work is not None:
+            return self._device_cycle()
         V, H, z, w = self.V, self.H, self.z, self.w
         for j in range(self.m):
             self._precondition(V[j], z)

@@ -399,6 +399,19 @@ int bw_r0_aca(int device, int64_t n_elems, const double *records, double G, doub
               double *factors_a, int64_t a_len, double *factors_b, int64_t b_len, int32_t *rank_out,
               double *err_out, void *stream);
 
+/* One Arnoldi step of GMRES after the operator, in four launches on `stream`:
+ * w (length n, the operator applied to the preconditioned V_j; overwritten) is
+ * orthogonalised against V_0 .. V_j (rows of length n of V, (m + 1) x n) by
+ * classical Gram-Schmidt with one re-orthogonalisation; column j of H
+ * ((m + 1) x m, row-major) receives the coefficients and |w|, V_{j+1} the
+ * normalised w.  |w| not above breakdown x the norm of the w passed in counts
+ * as zero: H(j + 1, j) = 0 and V_{j+1} = 0.  minv and z (both or neither null):
+ * z = minv * V_{j+1}.  work: 3 c (m + 2) doubles, c >= 1 (the CTAs used, at most
+ * one per SM).  Device pointers, FP64; stream-ordered, allocates nothing.
+ * The reference has no solver of its own. */
+int bw_arnoldi_step(int device, int64_t n, int j, int m, double *V, double *H, double *w, const double *minv,
+                    double *z, double *work, int64_t work_len, double breakdown, void *stream);
+
 /* Stresses and displacements at observation points from a solution on a
  * 2DS0 mesh (straight segments, constant displacement discontinuity, plane
  * strain): the device counterpart of BigWhamIO::ComputeStresses /
