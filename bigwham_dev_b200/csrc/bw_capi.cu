@@ -632,12 +632,13 @@ void launch_matvec_impl(bw_hmat *h, int o, int prec, const double *x, double *y,
   // 85.8 -> 75.7 us, a 256-segment crack 20.4 -> 17.0 us, 16,384 segments BF16
   // 54.8 -> 37.4 us.
   const bool early = !ev;
-  // The G2 gather beside an unstaged launch with a warp per unit, which fills
-  // the chip, costs more than its start-up (48 2DS0 cracks, BF16 141.4 against
-  // 132.3 us when it comes after; 20 cracks, FP32 68.1 against 58.5 us).
+  // The G2 gather beside an unstaged launch of one or two warps per unit, which
+  // fills the chip, costs more than its start-up: at once / after it, 48 2DS0
+  // cracks BF16 (1 warp) 141.4 / 132.3 us, 20 cracks FP32 (2 warps) 68.1 / 58.5
+  // us, 16,384 segments BF16 (4 warps) 37.4 / 39.6 us.
   const DevPhase &p1 = h->dev[o][prec][0];
   const bool early_g2 =
-      early && (p1.split.wide == p1.n_items || bw::narrow_team(p1.n_items - p1.split.coop, h->grid) > 1);
+      early && (p1.split.wide == p1.n_items || bw::narrow_team(p1.n_items - p1.split.coop, h->grid) > 2);
   if (n_in > 0) {
     bw::gather_x_kernel<G><<<(n_in + 255) / 256, 256, 0, st>>>(x, xp, xpk, perm_in, h->dof, n_in);
     BW_CUDA(cudaGetLastError());

@@ -288,8 +288,11 @@ __device__ __forceinline__ void chunk_dot<float, 4>(const unsigned char *base, c
 template <typename S> struct SmemLayout {
   using G = typename Store<S>::G;
   static constexpr int kDataBytes = kStageBytes + 32;
-  // vector window: the chunk's run of values with up to 15 bytes of slack each side
-  static constexpr int kGBytes = kMaxCols * (int)sizeof(G) + 32;
+  // vector window: the chunk's run of values with up to 15 bytes of slack each
+  // side (FP64 chunks have half the columns: a phase's unstaged CTAs then fit
+  // beside this kernel's)
+  static constexpr int kWindow = sizeof(G) == 8 ? kMaxColsFp64 : kMaxCols;
+  static constexpr int kGBytes = kWindow * (int)sizeof(G) + 32;
   static constexpr int kStageSize = kDataBytes + kGBytes + (int)sizeof(Chunk);
   static constexpr int kRedPer = Store<S>::kRed;
   static_assert(kHMax <= 2 * consumers_of<S>(), "each consumer thread writes at most two output rows of an item");
@@ -385,7 +388,7 @@ template <typename S> __device__ __forceinline__ unsigned long long chunk_bytes_
 }
 template <typename S> __device__ __forceinline__ bool chunk_ok(const uint32_t (&w)[kChunkWords]) {
   const int ncols = static_cast<int>(w[2]);
-  return ncols > 0 && ncols <= kMaxCols && chunk_bytes_of<S>(w) <= static_cast<unsigned long long>(kStageBytes);
+  return ncols > 0 && ncols <= SmemLayout<S>::kWindow && chunk_bytes_of<S>(w) <= static_cast<unsigned long long>(kStageBytes);
 }
 
 template <typename S>
@@ -621,7 +624,7 @@ __global__ void __launch_bounds__(threads_of<S>(), 1) stream_panels_kernel(Strea
 #pragma unroll
         for (int r = 0; r < R; r++) acc[r] = 0;
       }
-      if (active && ncols > 0 && ncols <= kMaxCols) {
+      if (active && ncols > 0 && ncols <= L::kWindow) {
         const int c0 = (cq * ncols) / Q, c1 = ((cq + 1) * ncols) / Q;
         const int soff = static_cast<int>((static_cast<unsigned long long>(d.data_off) * es) & 15ull);
         chunk_dot<S, R>(st + soff, gs, hv, rv, c0, c1, acc);
