@@ -2171,7 +2171,7 @@ int bw_arnoldi_step(int device, int64_t n, int j, int m, double *V, double *H, d
     int sms = 0;
     BW_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     const int grid = (int)std::max<int64_t>(
-        1, std::min<int64_t>({(int64_t)sms, (n + 63) / 64, work_len / (3 * (int64_t)(m + 2))}));
+        1, std::min<int64_t>({(int64_t)sms, (n + 127) / 128, work_len / (3 * (int64_t)(m + 2))}));
     bw::ArnoldiArgs a{V, H, w, minv, z, work, (long long)n, j, m, breakdown};
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const size_t smem = sizeof(double) * (size_t)(m + 2);

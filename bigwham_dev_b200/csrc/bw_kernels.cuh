@@ -307,6 +307,17 @@ struct DescRegs {
   uint32_t w[kChunkWords];
 };
 
+// x / q for 0 <= x < 2^17, 1 <= q <= 512: with m = ceil(2^32 / q) the product
+// x m / 2^32 exceeds x / q by less than 2^-15, and x / q is a multiple of 1 / q.
+// A chunk's column ranges take two such quotients by its item's q.
+struct SmallDivisor {
+  uint32_t m;
+  __device__ __forceinline__ void set(int q) { m = q > 1 ? 0xffffffffu / static_cast<uint32_t>(q) + 1u : 0u; }
+  __device__ __forceinline__ int divide(int x) const {
+    return m ? static_cast<int>(__umulhi(static_cast<uint32_t>(x), m)) : x;
+  }
+};
+
 template <int N> struct IntC {
   static constexpr int value = N;
 };
@@ -567,6 +578,7 @@ __global__ void __launch_bounds__(threads_of<S>(), 1) stream_panels_kernel(Strea
   // FMA path state
   constexpr int R = kTensor ? 1 : Store<S>::kRows;
   int hv = 1, Q = 1, rv = 0, cq = 0;
+  SmallDivisor by_q{0u};
   bool active = false;
   G acc[R];
 #pragma unroll
@@ -618,6 +630,7 @@ __global__ void __launch_bounds__(threads_of<S>(), 1) stream_panels_kernel(Strea
       if (flags & kFirst) {
         hv = hpad / R;
         Q = kConsumers / hv;
+        by_q.set(Q);
         rv = ct % hv;
         cq = ct / hv;
         active = cq < Q;
@@ -625,7 +638,7 @@ __global__ void __launch_bounds__(threads_of<S>(), 1) stream_panels_kernel(Strea
         for (int r = 0; r < R; r++) acc[r] = 0;
       }
       if (active && ncols > 0 && ncols <= L::kWindow) {
-        const int c0 = (cq * ncols) / Q, c1 = ((cq + 1) * ncols) / Q;
+        const int c0 = by_q.divide(cq * ncols), c1 = by_q.divide((cq + 1) * ncols);
         const int soff = static_cast<int>((static_cast<unsigned long long>(d.data_off) * es) & 15ull);
         chunk_dot<S, R>(st + soff, gs, hv, rv, c0, c1, acc);
       }

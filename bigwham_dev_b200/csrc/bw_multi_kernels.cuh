@@ -313,6 +313,7 @@ __global__ void __launch_bounds__(threads_of<S>(), 1) stream_multi_kernel(MultiA
   long long pre_dst[kPre];
   uint32_t items = 0;
   int hv = 1, Q = 1, rv = 0, cq = 0;
+  SmallDivisor by_q{0u};
   bool active = false;
   G acc[R][K];
 #pragma unroll
@@ -338,6 +339,7 @@ __global__ void __launch_bounds__(threads_of<S>(), 1) stream_multi_kernel(MultiA
     if (flags & kFirst) {
       hv = hpad / R;
       Q = kConsumers / hv;
+      by_q.set(Q);
       rv = ct % hv;
       cq = ct / hv;
       active = cq < Q;
@@ -352,7 +354,7 @@ __global__ void __launch_bounds__(threads_of<S>(), 1) stream_multi_kernel(MultiA
       }
     }
     if (active && ncols > 0 && ncols <= L::kCols) {
-      const int c0 = (cq * ncols) / Q, c1 = ((cq + 1) * ncols) / Q;
+      const int c0 = by_q.divide(cq * ncols), c1 = by_q.divide((cq + 1) * ncols);
       const int soff = static_cast<int>((static_cast<unsigned long long>(d.data_off) * es) & 15ull);
       chunk_dot_multi<G, R, K>(st + soff, gs, hv, rv, c0, c1, acc);
     }
