@@ -4,8 +4,9 @@ The reference computes stresses and displacements at arbitrary points from a
 displacement-discontinuity solution on the host (BigWhamIO::ComputeStresses /
 ComputeDisplacements, src/io/bigwham_io.cc:1166-1324): a dense loop over
 (source element, observation point) pairs, OpenMP over the source points.
-Here the same dense sum runs in ``bw_s0_fields`` (one thread per observation
-point, elements in mesh order; bw_s0.h holds the element's closed forms).
+Here the same dense sum runs in ``bw_s0_fields`` (1 to 32 lanes per observation
+point, each over every lanes-th element in mesh order; bw_s0.h holds the
+element's closed forms).
 
 2DS0 (``S0Fields``, bw_s0_fields): per point (s11, s22, s12) and (u1, u2),
 global frame, from the local DD per element (shear, normal), mesh order.

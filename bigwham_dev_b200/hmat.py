@@ -310,7 +310,9 @@ class HmatGpu:
         X and Y are column-major (each right-hand side contiguous); X is copied
         to that layout when it is not.  "bf16" on a handle finalized with
         matmat=True runs on the tensor cores, 64 right-hand sides per pass;
-        everything else applies one matvec per column."""
+        "fp64" and "fp32" read the blocks once per 8 columns (each column equal
+        to its matvec bit for bit); everything else applies one matvec per
+        column."""
         import torch
 
         nin, nout = (self.n_rows, self.n_cols) if transpose else (self.n_cols, self.n_rows)

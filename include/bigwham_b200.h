@@ -203,7 +203,7 @@ int bw_matvec_static_scratch(bw_hmat *h, const double *x, double *y, int flags, 
 
 /* Same product on HOST arrays: copies x to the device, runs bw_matvec on the
  * handle's stream, copies y back and synchronizes.  The vectors move in four
- * pieces through pinned buffers of the handle, so the host copies overlap
+ * pieces (one below 65,536 values) through pinned buffers of the handle, so the host copies overlap
  * the DMA; on BW_ERR_DEVICE the contents of y are unspecified.
  * Replaces: Hmat<double>::matvecOriginal(il::ArrayView<double>) / matvec(...)
  * (hmat.cc:572-635 / :472-537), reached from BigWhamIO::MatVec(il::ArrayView)
@@ -216,8 +216,11 @@ int bw_matvec_host(bw_hmat *h, const double *x, double *y, int flags);
  * tensor cores:
  *  - X is rounded to BF16, products accumulate in FP32;
  *  - 64 right-hand sides per pass of 3 launches.
- * Otherwise it is one bw_matvec per column.  BW_PERMUTED and BW_TRANSPOSE
- * apply as for bw_matvec.  No reference counterpart. */
+ * With BW_FP64 or BW_FP32 the block data is read once per 8 (or 4) columns; each
+ * column equals its bw_matvec bit for bit.  Otherwise (BF16 without that
+ * layout, per-launch timing, narrow_coop, X and Y ranges that interleave, no
+ * device memory for the scratch at bw_finalize) it is one bw_matvec per column.
+ * BW_PERMUTED and BW_TRANSPOSE apply as for bw_matvec.  No reference counterpart. */
 int bw_matmat(bw_hmat *h, const double *X, int64_t ldx, double *Y, int64_t ldy, int nrhs, int flags,
               void *stream);
 
@@ -420,8 +423,9 @@ int bw_arnoldi_step(int device, int64_t n, int j, int m, double *V, double *H, d
  * length, unit tangent x, y, the tangent running from the first vertex to the
  * second); dd: n_elems x 2 local DDs (shear, normal), mesh order; pts:
  * n_pts x 2; stress (n_pts x 3: s11, s22, s12) and / or disp (n_pts x 2,
- * global frame) may be null, not both.  Each point sums the elements in mesh
- * order.  Stream-ordered; returns after the launch. */
+ * global frame) may be null, not both.  Each point sums the elements in a fixed
+ * order (1 to 32 interleaved sums, each in mesh order).  Stream-ordered; returns
+ * after the launch. */
 int bw_s0_fields(int device, int64_t n_elems, const double *records, const double *dd, double G, double nu,
                  int64_t n_pts, const double *pts, double *stress, double *disp, void *stream);
 
