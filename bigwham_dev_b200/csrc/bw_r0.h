@@ -36,9 +36,9 @@
 //   F_z = -atan(X Y / (z R))                         F_xz = z / (R (R + Y))
 //   F_zz = X Y (X^2 + Y^2 + 2 z^2) / (R (X^2 + z^2) (Y^2 + z^2))
 //   F_xxy = -X / R^3      F_xyz = -z / R^3
-//   F_xxx = d/dX F_xx     F_xxz = d/dz F_xx          F_xzz = d/dz F_xz
-// (y forms by X <-> Y), and I_zzz = -(I_xxz + I_yyz) (I is harmonic off the
-// plane).  Numerics:
+//   F_xxx = d/dX F_xx     F_xxz = d/dz F_xx
+// (y forms by X <-> Y), and I_zzz = -(I_xxz + I_yyz), I_xzz = -(I_xxx + I_xyy),
+// I_yzz = -(I_yyy + I_xxy) (I is harmonic off the plane).  Numerics:
 // * R + Y cancels when Y < 0 and X^2 + z^2 << Y^2, so it is evaluated as
 //   (X^2 + z^2) / (R - Y) there (an identity);
 // * in the element plane (z == 0) I_xz = I_yz = 0, I_zz = -(I_xx + I_yy),
@@ -92,8 +92,10 @@ BW_HD double refine_inv(double v, double r) { return fma(r, fma(-v, r, 1.0), r);
 // one for the two X^2 + z^2, one for the two Y^2 + z^2 and one per corner for
 // 1 / (R + |X|) and 1 / (R + |Y|) together (some 80 with every term by itself).  With P = R (R + Y), p = 1 / P and
 // k = 2 + Y / R:
-//   F_xx = X p, F_xz = z p, F_xxx = (P - X^2 k) p^2, F_xzz = (P - z^2 k) p^2,
-//   F_xxz = -X z k p^2.
+//   F_xx = X p, F_xz = z p, F_xxx = (P - X^2 k) p^2, F_xxz = -X z k p^2.
+// I_xzz and I_yzz come from the others: fewer operations, and against extended
+// precision a smaller error than with corner terms of their own (median over
+// points around meshes of 72 to 2,000 elements 3.5e-15, 4.1e-15 with them).
 BW_HD Derivs derivs_offplane(double x, double y, double z, double a, double b) {
   Derivs d = {};
   const double Xc[2] = {x + a, x - a}, Yc[2] = {y + b, y - b};
@@ -141,8 +143,6 @@ BW_HD Derivs derivs_offplane(double x, double y, double z, double a, double b) {
       d.yyy += s * ((Q - Y * Y * kq) * q2);
       d.xxz -= s * (X * kp * p2);
       d.yyz -= s * (Y * kq * q2);
-      d.xzz += s * ((P - z2 * kp) * p2);
-      d.yzz += s * ((Q - z2 * kq) * q2);
     }
     d.z -= atan2(im, re);
   }
@@ -154,7 +154,9 @@ BW_HD Derivs derivs_offplane(double x, double y, double z, double a, double b) {
   d.xyz *= z;
   d.xxz *= z;
   d.yyz *= z;
-  d.zzz = -(d.xxz + d.yyz);
+  d.zzz = -(d.xxz + d.yyz);  // harmonic
+  d.xzz = -(d.xxx + d.xyy);
+  d.yzz = -(d.yyy + d.xxy);
   return d;
 }
 
