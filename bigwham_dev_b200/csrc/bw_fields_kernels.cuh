@@ -29,7 +29,7 @@ constexpr int kFieldTile = 128;     // elements per shared-memory tile
 // Lanes per point: the fewest (a power of two up to a warp) that give a call
 // two threads for each of 1,024 per SM.  2DS0, 4,000 segments: 50,000 points
 // 8.05 -> 2.46 ms with the element's combined forms, 300 to 1,000 points up to
-// 60 times faster; 3DR0, 4,096 elements, 20,000 points 36.0 -> 4.54 ms.
+// 60 times faster; 3DR0, 4,096 elements, 20,000 points 36.0 -> 4.52 ms.
 constexpr long long kFieldThreadsWanted = 2LL * 148 * 1024;
 
 inline int field_lanes(long long n_pts) {
