@@ -121,6 +121,10 @@ __device__ __forceinline__ void bulk_g2s_hint(void *dst, const void *src, uint32
 // one has issued launch_dependents (or exited); wait blocks until the grids
 // this one depends on have completed and their writes are visible.  Both are
 // no-ops without such a launch.
+// What a launch before it writes (gathered x, t, G2) a kernel that may start
+// early reads through the async proxy or with ordinary loads, never as read-only
+// data (__ldg, const __restrict__ parameters): read-only loads presume that
+// nobody writes the data while the kernel is resident, and may pass the wait.
 __device__ __forceinline__ void pdl_launch_dependents() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
@@ -571,6 +575,9 @@ __global__ void __launch_bounds__(threads_of<S>(), 1) stream_panels_kernel(Strea
   }
 
   // -------------------------------------------------------------------- consumers
+  // Nothing is staged before the launch in front of this one is done: the wait
+  // limit counts from there.
+  pdl_wait();
   const int ct = threadIdx.x - 32;
   const int cw = warp - 1;
   uint32_t items = 0;
@@ -867,7 +874,7 @@ __device__ __forceinline__ void narrow_fma_chunk(const unsigned char *base, cons
       const int cq = c + q * cpp;
       if (cq < ncols) {
         v[q] = __ldg(reinterpret_cast<const V *>(d + static_cast<long long>(cq) * hpad));
-        x[q] = __ldg(g + cq);
+        x[q] = g[cq];
       } else {
         v[q] = V{};
         x[q] = 0;
@@ -917,7 +924,7 @@ __device__ __forceinline__ void narrow_bf16_chunk_t(const uint16_t *base, const 
       const int cq = cg + q * gpw, c = 8 * cq + c8;
       const bool in = cq < ncg && c < ncols;  // the tile's padding columns are not read
       const uint16_t *col = lb + static_cast<long long>(cq) * 8 * hpad;
-      x[q] = in ? unpack_hilo(__ldg(g + c)) : 0.f;
+      x[q] = in ? unpack_hilo(g[c]) : 0.f;
       w[q][0] = in && one ? __ldg(reinterpret_cast<const uint4 *>(col)) : make_uint4(0, 0, 0, 0);
       if constexpr (kTwo) w[q][1] = in && two ? __ldg(reinterpret_cast<const uint4 *>(col + 256)) : make_uint4(0, 0, 0, 0);
     }
@@ -1222,8 +1229,7 @@ inline int g2_runs_per_warp(long long n_runs, int sms) {
 
 template <typename G, bool kPacked>
 __global__ void gather_g2_kernel(const GatherSeg *__restrict__ runs, int n_runs, int per_warp,
-                                 const G *__restrict__ xp,
-                                 const G *__restrict__ t, void *__restrict__ g2) {
+                                 const G *xp, const G *t, void *g2) {
   const int lane = threadIdx.x & 31;
   const int r0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * per_warp;
   if (r0 >= n_runs) {  // warp-uniform

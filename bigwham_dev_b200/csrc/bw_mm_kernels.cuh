@@ -184,6 +184,10 @@ __global__ void __launch_bounds__(kMmThreads, 1) mm_stream_kernel(MmArgs a) {
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
+  // Nothing is staged before the launch in front of this one is done: the wait
+  // limit of the issuers and the epilogue counts from there.
+  if (warp != 0) pdl_wait();
+
   if (warp == 0) {
     // ------------------------------------------------------------------ producer
     const unsigned char *gdata = reinterpret_cast<const unsigned char *>(a.data);

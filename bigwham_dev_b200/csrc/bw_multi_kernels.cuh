@@ -305,6 +305,7 @@ __global__ void __launch_bounds__(threads_of<S>(), 1) stream_multi_kernel(MultiA
   }
 
   // -------------------------------------------------------------------- consumers
+  pdl_wait();  // as in stream_panels_kernel: the wait limit counts from here
   const int ct = threadIdx.x - 32, cw = warp - 1;
   // phase 2 output rows of this thread: row0, row0 + kRowStep, ...; the first
   // kPre places in y are loaded at an item's first chunk

@@ -88,7 +88,8 @@ int bw_batch_offsets(const bw_hmat *h, int member, int64_t *row0, int64_t *col0)
 int bw_batch_count(const bw_hmat *h);
 
 /* Bound (in ns, 1 ns .. 60 s, default 2 s) of every wait inside the kernels:
- * a stage that never fills or empties, an item reduction that never completes.
+ * a stage that never fills or empties, an item reduction that never completes
+ * (counted once the launch before this one is done).
  * When a wait runs out the kernel writes an error word and returns; the
  * cleanup waits (copies in flight, tensor-core work before its memory is
  * freed) keep their own 2 s bound, so no work is left outstanding.  The next

@@ -9,7 +9,8 @@ one chunk: a barrier that nothing completes.  With a 20 ms wait limit
 * frees its TMEM and returns.
 The next sync reports BW_ERR_DEVICE.  With the default limit restored the same
 handle gives the bitwise-same results as before: no state is left behind
-(error word, work-queue counters, TMEM).
+(error word, work-queue counters, TMEM).  The limit counts from the end of the
+launch before: a product whose phase 1 takes longer than the limit is healthy.
 """
 import numpy as np
 import pytest
@@ -59,3 +60,33 @@ def test_wait_limit_range_checked(handle):
         with pytest.raises(BigWhamError) as e:
             handle.set_wait_limit(bad)
         assert e.value.status == A.BW_ERR_ARG
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+def test_the_limit_is_a_stage_s_not_the_launch_before_s(prec):
+    """A phase-2 CTA may get its SM while phase 1 still runs elsewhere (here on
+    one CTA: a single item of a million columns) and waits for it.  That wait
+    does not count: a limit well below the phase's time, and well above any
+    stage's, reports nothing."""
+    import torch
+
+    n, m, k, limit_us = 1 << 20, 64, 8, 300
+    rng = np.random.default_rng(0)
+    h = HmatGpu(1, m, n, np.arange(m), np.arange(n), device=0).set_tuning(narrow_rows=0)
+    h.add_lowrank(0, 0, rng.uniform(-1, 1, (m, 1)), rng.uniform(-1, 1, (1, n)))
+    h.finalize(precisions=(prec,))
+    X = torch.from_numpy(rng.uniform(-1, 1, (k, n))).cuda().t()
+    want, want1 = h.matmat(X, prec).clone(), h.matvec(X[:, 0], prec).clone()
+    ev = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+    h.sync()
+    ev[0].record()
+    h.matmat(X, prec)
+    ev[1].record()
+    h.sync()
+    assert ev[0].elapsed_time(ev[1]) > 2e-3 * limit_us  # else the limit tests nothing
+    h.set_wait_limit(1000 * limit_us)
+    for _ in range(5):
+        Y, y = h.matmat(X, prec), h.matvec(X[:, 0], prec)
+        h.sync()
+        assert torch.equal(Y, want) and torch.equal(y, want1)
+    h.close()
