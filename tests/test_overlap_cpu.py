@@ -47,5 +47,6 @@ def test_vectors_are_read_with_coherent_loads(file, function, read):
                                            ("bw_mm_kernels.cuh", "mm_stream_kernel")])
 def test_bulk_copies_come_after_a_proxy_fence(file, function):
     _, body = _body(file, function)
-    wait = body.index("pdl_wait();")
-    assert re.match(r"pdl_wait\(\);\s*fence_proxy_async_global\(\);\s*pdl_launch_dependents\(\);", body[wait:])
+    fence = r"pdl_wait\(\);\s*fence_proxy_async_global\(\);\s*pdl_launch_dependents\(\);"
+    assert len(re.findall(fence, body)) == 1
+    assert len(re.findall(r"fence_proxy_async_global|pdl_launch_dependents", body)) == 2
