@@ -58,6 +58,7 @@ _SIGS = {
     "bw_plan_tscale": (C.c_int, [_P, C.c_int, _P, _P]),
     "bw_mm_plan_export": (C.c_int, [_P, C.c_int, C.c_int, _P, _P, _P, _P, _P, _P, _P]),
     "bw_plan_gather": (C.c_int, [_P, C.c_int, C.c_int, _P, _P]),
+    "bw_plan_slices": (C.c_int, [_P, C.c_int, C.c_int, _P, _P, _P, _P, _P]),
     "bw_file_write": (C.c_int, [C.c_char_p, C.c_int, _I64, _I64, _P, _P, _I64, _P, _P, _I64, _P, _P, _P]),
     "bw_file_write_blocks": (C.c_int, [C.c_char_p, C.c_int, _I64, _I64, _P, _P, _I64, _P, _P, _P, _I64, _P, _P, _P,
                                        _P, _P, _P]),

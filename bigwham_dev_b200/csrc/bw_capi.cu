@@ -503,6 +503,20 @@ bw::NarrowSplit narrow_split(const bw::ChunkPlan &cp, const bw::Tuning &tune, in
   return sp;
 }
 
+// f(i, place) for every phase-2 chunk i, with a slice of the gather array for
+// each (the plan shares slices between the row parts of a panel); false when a
+// place passes the 32 bits that the exports give it.
+template <typename F> bool each_slice(const bw::ChunkPlan &cp, F &&f) {
+  int64_t len = 0;
+  for (size_t i = 0; i < cp.chunks.size(); i++) {
+    const int64_t g = (len + 3) / 4 * 4;
+    len = g + cp.chunks[i].ncols;
+    if (len > INT32_MAX) return false;
+    f(i, g);
+  }
+  return true;
+}
+
 // Upload the data of one phase in pieces through two pinned staging buffers.
 void upload_phase(bw_hmat *h, int o, int prec, int phase) {
   const bw::OperatorPlan &op = h->op[o];
@@ -1587,11 +1601,9 @@ int bw_plan_export(const bw_hmat *h, int precision, int phase, int transposed, i
   if (n_item_ptr) *n_item_ptr = (int64_t)cp.item_ptr.size();
   if (chunks) {
     std::memcpy(chunks, cp.chunks.data(), cp.chunks.size() * sizeof(Chunk));  // kChunkWords int32 each
-    if (phase == 2) {
-      const std::vector<int32_t> g_off = bw::slice_per_chunk(cp).g_off;
-      for (size_t i = 0; i < g_off.size(); i++)
-        std::memcpy(chunks + i * bw::kChunkWords + offsetof(Chunk, g_off) / 4, &g_off[i], 4);
-    }
+    int32_t *g_off = chunks + offsetof(Chunk, g_off) / 4;
+    if (phase == 2 && !each_slice(cp, [&](size_t i, int64_t g) { g_off[i * bw::kChunkWords] = (int32_t)g; }))
+      return BW_ERR_UNSUPPORTED;
   }
   if (item_ptr) std::memcpy(item_ptr, cp.item_ptr.data(), cp.item_ptr.size() * sizeof(int32_t));
   if (data) {
@@ -1704,9 +1716,39 @@ int bw_plan_gather(const bw_hmat *h, int precision, int transposed, int64_t *n, 
   if (p < 0 || !h->finalized || !(h->stored & (1 << p))) return BW_ERR_STATE;
   const int o = transposed ? 1 : 0;
   if (o == 1 && !h->has_t) return BW_ERR_UNSUPPORTED;
-  const std::vector<bw::GatherSeg> g = bw::slice_per_chunk(h->op[o].ph[1].cp[p]).gsegs;
-  *n = (int64_t)g.size();
-  if (runs) std::memcpy(runs, g.data(), g.size() * sizeof(bw::GatherSeg));
+  const bw::ChunkPlan &cp = h->op[o].ph[1].cp[p];
+  int64_t k = 0;
+  const bool fits = each_slice(cp, [&](size_t i, int64_t g) {
+    for (int32_t q = 0; q < cp.ranges[i].second; q++, k++) {
+      if (!runs) continue;
+      bw::GatherSeg s = cp.gsegs[cp.ranges[i].first + q];
+      s.dst = (int32_t)(g + (s.dst - cp.chunks[i].g_off));
+      std::memcpy(runs + 4 * k, &s, sizeof s);
+    }
+  });
+  if (!fits) return BW_ERR_UNSUPPORTED;
+  *n = k;
+  return BW_OK;
+}
+
+int bw_plan_slices(const bw_hmat *h, int precision, int transposed, int64_t *g_len, int64_t *n_chunks, int32_t *slices,
+                   int64_t *n_runs, int32_t *runs) {
+  if (!h || !g_len || !n_chunks || !n_runs) return BW_ERR_ARG;
+  const int p = prec_index(precision);
+  if (p < 0 || !h->finalized || !(h->stored & (1 << p))) return BW_ERR_STATE;
+  const int o = transposed ? 1 : 0;
+  if (o == 1 && !h->has_t) return BW_ERR_UNSUPPORTED;
+  const bw::ChunkPlan &cp = h->op[o].ph[1].cp[p];
+  *g_len = cp.g_len;
+  *n_chunks = (int64_t)cp.chunks.size();
+  *n_runs = (int64_t)cp.gsegs.size();
+  if (slices)
+    for (size_t i = 0; i < cp.chunks.size(); i++) {
+      slices[3 * i] = cp.chunks[i].g_off;
+      slices[3 * i + 1] = cp.ranges[i].first;
+      slices[3 * i + 2] = cp.ranges[i].second;
+    }
+  if (runs && !cp.gsegs.empty()) std::memcpy(runs, cp.gsegs.data(), cp.gsegs.size() * sizeof(bw::GatherSeg));
   return BW_OK;
 }
 

@@ -508,22 +508,6 @@ void build_chunks(const Problem &p, bool tr, int prec, int grid, OperatorPlan &o
   }
 }
 
-ChunkSlices slice_per_chunk(const ChunkPlan &cp) {
-  ChunkSlices out;
-  int64_t len = 0;
-  for (size_t i = 0; i < cp.ranges.size(); i++) {
-    const int64_t g = (len + 3) / 4 * 4;
-    out.g_off.push_back(i32(g, "G2 offset"));
-    for (int32_t k = 0; k < cp.ranges[i].second; k++) {
-      GatherSeg s = cp.gsegs[cp.ranges[i].first + k];
-      s.dst = i32(g + (s.dst - cp.chunks[i].g_off), "G2 offset");
-      out.gsegs.push_back(s);
-    }
-    len = g + cp.chunks[i].ncols;
-  }
-  return out;
-}
-
 namespace {
 
 // One column run of an item: rows [r0, r0 + n) of item column c from

@@ -131,20 +131,12 @@ struct ChunkPlan {
   std::vector<int32_t> item_ptr;  // queue units + 1 (chunk index of each unit's first chunk)
   std::vector<GatherSeg> gsegs;   // phase 2 only
   // phase 2: each chunk's runs in gsegs (first, count), in the chunks' order;
-  // they tile the chunk's vector values in order
+  // they tile the chunk's vector values in order.  The row parts of one panel
+  // multiply the same vector values, and those of equal height are cut into the
+  // same columns, so they share their slices of G2 and their runs.
   std::vector<std::pair<int32_t, int32_t>> ranges;
   int64_t g_len = 0;
 };
-
-// A phase-2 plan with a slice of G2 for every chunk, as the plan export shows
-// it.  The plan itself shares: the row parts of one panel multiply the same
-// vector values, and those of equal height are cut into the same columns, so
-// they read one slice.
-struct ChunkSlices {
-  std::vector<int32_t> g_off;     // per chunk
-  std::vector<GatherSeg> gsegs;
-};
-ChunkSlices slice_per_chunk(const ChunkPlan &cp);
 
 struct PhasePlan {
   std::vector<Item> items;

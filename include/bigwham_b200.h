@@ -273,8 +273,9 @@ int bw_mm_plan_export(const bw_hmat *h, int phase, int transposed, int64_t *n_ch
  * FP32, 8x8 tiles for BF16; BF16 values divided by their block scale);
  * item_ptr: the chunk ranges of the items (n_item_ptr = items + 1 offsets), in
  * the order the kernel's CTAs take them (longest first).  Phase 2 is shown with
- * a slice of the gather array for every chunk; on the device the row parts of
- * one panel share theirs.  data is only available on a handle finalized with
+ * a slice of the gather array for every chunk (BW_ERR_UNSUPPORTED past 2^31
+ * values); on the device the row parts of one panel share theirs
+ * (bw_plan_slices).  data is only available on a handle finalized with
  * BW_PLAN_ONLY. */
 int bw_plan_export(const bw_hmat *h, int precision, int phase, int transposed, int64_t *n_chunks,
                    int32_t *chunks, int64_t *n_elems, double *data, int64_t *n_item_ptr, int32_t *item_ptr);
@@ -310,6 +311,13 @@ int bw_phase_bytes(const bw_hmat *h, int precision, int transposed, int64_t *pha
 /* Runs that fill the phase-2 gather array (4 int32 words each: dst, src_off,
  * cols | src << 31, scale bits), for inspection and testing. */
 int bw_plan_gather(const bw_hmat *h, int precision, int transposed, int64_t *n, int32_t *runs);
+
+/* Phase 2's vector values as the device reads them: g_len, the length of the
+ * gather array; per chunk (n_chunks x 3) its place in that array, its first run
+ * and its number of runs, which fill the slice in order; the runs as in
+ * bw_plan_gather, without the repetitions.  slices and runs may be NULL. */
+int bw_plan_slices(const bw_hmat *h, int precision, int transposed, int64_t *g_len, int64_t *n_chunks, int32_t *slices,
+                   int64_t *n_runs, int32_t *runs);
 
 /* Per-t-entry scales of the BF16 layout (scale(A) * scale(B) of the entry's
  * low-rank block; 1 elsewhere), for inspection and testing.  Phase 1 writes t

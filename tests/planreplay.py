@@ -67,16 +67,39 @@ def build_g2(runs, x, t):
     return g2
 
 
-def replay(h, x_perm, precision="fp64", transposed=False):
-    """y (permuted ordering) = H x_perm, replaying h's plan (h finalized with plan_only)."""
+def slices(h, precision, transposed):
+    """Phase 2's vector values as the device reads them: (length of G2, per
+    chunk [place in G2, first run, runs], the runs)."""
     from bigwham_dev_b200 import _capi as A
 
+    g, nc, nr = C.c_int64(), C.c_int64(), C.c_int64()
+    f = A.PRECISIONS[precision]
+    A.check(A.lib().bw_plan_slices(h._h, f, int(transposed), C.byref(g), C.byref(nc), None, C.byref(nr), None), h._h)
+    sl, runs = np.zeros((nc.value, 3), np.int32), np.zeros((nr.value, 4), np.int32)
+    A.check(A.lib().bw_plan_slices(h._h, f, int(transposed), C.byref(g), C.byref(nc), sl.ctypes.data, C.byref(nr),
+                                   runs.ctypes.data), h._h)
+    return g.value, sl, runs
+
+
+def device_phase2(h, precision, transposed, with_data=True):
+    """Phase 2's plan with the places in G2 and the runs that the device uses
+    (plan_export and gather_runs show a slice for every chunk)."""
+    p2 = h.plan_export(precision, 2, transposed, with_data=with_data)
+    g_len, sl, runs = slices(h, precision, transposed)
+    p2["chunks"][:, 7] = sl[:, 0]
+    return p2, runs, g_len
+
+
+def replay(h, x_perm, precision="fp64", transposed=False):
+    """y (permuted ordering) = H x_perm, replaying h's plan (h finalized with
+    plan_only) as the device runs it."""
     p1 = h.plan_export(precision, 1, transposed)
-    p2 = h.plan_export(precision, 2, transposed)
+    p2, runs, g_len = device_phase2(h, precision, transposed)
     tiled = precision == "bf16"
     t = np.zeros(max(1, h.info()["sum_rank"]))
     run_phase(p1, x_perm, t, tiled)  # BF16: t unscaled; the G2 runs carry the block scales
-    g2 = build_g2(gather_runs(h, precision, transposed), x_perm, t)
+    g2 = build_g2(runs, x_perm, t)
+    assert g2.size <= g_len
     y = np.full(h.n_cols if transposed else h.n_rows, np.nan)
     run_phase(p2, g2, y, tiled)
     return y

@@ -16,7 +16,7 @@ H and H^T, every precision within its rounding bound.
 """
 import numpy as np
 import pytest
-from planreplay import build_g2, decode, gather_runs, run_phase
+from planreplay import build_g2, decode, device_phase2, run_phase
 
 from bigwham_dev_b200 import HmatGpu
 from oracle import oracle_matvec_perm, oracle_rmatvec_perm
@@ -121,10 +121,10 @@ def split_phase(plan, gsrc, out, precision, rows=NARROW_ROWS, coop=0):
 
 def narrow_replay(h, x_perm, precision, transposed=False, rows=NARROW_ROWS, coop=0):
     p1 = h.plan_export(precision, 1, transposed)
-    p2 = h.plan_export(precision, 2, transposed)
+    p2, runs, _ = device_phase2(h, precision, transposed)
     t = np.zeros(max(1, h.info()["sum_rank"]))
     s1 = split_phase(p1, x_perm, t, precision, rows, coop)
-    g2 = build_g2(gather_runs(h, precision, transposed), x_perm, t)
+    g2 = build_g2(runs, x_perm, t)
     y = np.full(h.n_cols if transposed else h.n_rows, np.nan)
     s2 = split_phase(p2, g2, y, precision, rows, coop)
     return y, (s1, s2)
