@@ -829,10 +829,9 @@ void alloc_multi(bw_hmat *h, int mask, bool with_t) {
 
 // Whether a product of several columns can run in the multi-column kernels:
 // their scratch is there, no unit runs CTA-cooperatively (narrow_coop), and
-// neither per-launch timing nor the withheld-chunk test hook is asked for
-// (both belong to the matvec's launches).
+// per-launch timing (of the matvec's launches) is not asked for.
 bool multi_ready(const bw_hmat *h, int o, int prec) {
-  if (prec > 1 || !h->d_xk || !h->d_tk || h->timing || h->withhold >= 0) return false;
+  if (prec > 1 || !h->d_xk || !h->d_tk || h->timing) return false;
   if (h->dev[o][prec][1].n_chunks == 0 || !h->dev[o][prec][1].ranges) return false;
   for (const DevPhase &dp : h->dev[o][prec])
     if (dp.split.coop > dp.split.wide) return false;
@@ -869,6 +868,7 @@ void launch_multi(bw_hmat *h, int o, int prec, const double *X, int64_t ldx, dou
     m.s.phase = phase + 1;
     m.s.err = h->d_err;
     m.s.spin_limit = h->spin_limit;
+    m.s.withhold = h->take_withhold();  // the test hook applies to phase 1
     m.xk = h->d_xk;
     m.tk = h->d_tk;
     m.runs = dp.gsegs;

@@ -164,6 +164,8 @@ __global__ void __launch_bounds__(threads_of<S>(), 1) stream_multi_kernel(MultiA
     const unsigned char *gx = static_cast<const unsigned char *>(m.xk);
     const unsigned char *gt = static_cast<const unsigned char *>(m.tk);
     constexpr uint32_t kRowBytes = K * (uint32_t)sizeof(G);
+    // test hook: a withheld chunk of phase 1 is never staged, so its wait runs out
+    const int hold = a.phase == 1 && blockIdx.x == 0 ? a.withhold : -1;
     bool ok = true;
     int issued = 0;
     ItemQueue iq;
@@ -228,7 +230,7 @@ __global__ void __launch_bounds__(threads_of<S>(), 1) stream_multi_kernel(MultiA
           }
           good = __all_sync(0xffffffffu, in) && __reduce_add_sync(0xffffffffu, cols) == ncols;
         }
-        if (lane == 0) {
+        if (lane == 0 && issued != hold) {
           uint4 *dd = reinterpret_cast<uint4 *>(st + L::kDataBytes + L::kGBytes);
 #pragma unroll
           for (int q = 0; q < kChunkWords / 4; q++)
@@ -290,8 +292,11 @@ __global__ void __launch_bounds__(threads_of<S>(), 1) stream_multi_kernel(MultiA
       }
     }
     if (!ok) {
-      for (int i = max(0, issued - kSt); i < issued; i++)
+      // let the copies already in flight land before the CTA can exit
+      for (int i = max(0, issued - kSt); i < issued; i++) {
+        if (i == hold) continue;  // nothing in flight for it
         mbar_wait(&full[i % kSt], static_cast<uint32_t>(i / kSt) & 1u, kDrainLimitNs);
+      }
     }
     if (lane == 0) {
       __threadfence();

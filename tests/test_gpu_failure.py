@@ -63,6 +63,40 @@ def test_wait_limit_range_checked(handle):
 
 
 @pytest.mark.parametrize("prec", ["fp64", "fp32"])
+def test_timeout_of_several_columns(prec):
+    """The same for the products of several columns (passes of 8 and 4): some
+    nine items per CTA in phase 1, all of them CTA-wide."""
+    import torch
+
+    nb, bs, r = 64, 64, 8
+    n = nb * bs
+    rng = np.random.default_rng(0)
+    h = HmatGpu(1, n, n, np.arange(n), np.arange(n), device=0).set_tuning(narrow_rows=0)
+    fr = np.zeros((0, 4), np.int64)
+    lr = np.array([(i * bs, j * bs, (i + 1) * bs, (j + 1) * bs, r) for i in range(nb) for j in range(nb)], np.int64)
+    h.add_flat(fr, lr, np.zeros(0), rng.standard_normal(nb * nb * 2 * r * bs))
+    h.finalize(precisions=(prec,))
+    X, other = (torch.from_numpy(rng.uniform(-1, 1, (8, n))).cuda().t() for _ in range(2))
+    good = {k: h.matmat(X[:, :k], prec).clone() for k in (8, 3)}
+    h.sync()
+    for k in good:
+        h.set_wait_limit(20_000_000)
+        h.matmat(other[:, :k], prec)  # what the lost chunk's products are then replaced by
+        A.check(A.lib().bw_test_withhold_chunk(h._h, 1), h._h)
+        Y = h.matmat(X[:, :k], prec)
+        with pytest.raises(BigWhamError) as e:
+            h.sync()
+        assert e.value.status == A.BW_ERR_DEVICE and "error word" in str(e.value)
+        # one pass holds all columns, so the chunk is lost to each of them
+        assert not any(torch.equal(Y[:, j], good[k][:, j]) for j in range(k))
+        h.set_wait_limit(2_000_000_000)
+        for q in good:
+            assert torch.equal(h.matmat(X[:, :q], prec), good[q])
+        h.sync()
+    h.close()
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
 def test_the_limit_is_a_stage_s_not_the_launch_before_s(prec):
     """A phase-2 CTA may get its SM while phase 1 still runs elsewhere (here on
     one CTA: a single item of a million columns) and waits for it.  That wait

@@ -5,7 +5,8 @@ The multi-column kernels keep the matvec's arithmetic order in every column,
 so each column must equal the matvec of that column bit for bit; the matvec
 itself is checked against the oracle elsewhere.  Counts of columns around the
 passes' edges (a single one left over, up to 4, up to 8), both kernels of the
-phase split, ragged partitions, rank-0 blocks, H and H^T, both orderings and
+phase split (with narrow_coop 1 units run CTA-cooperatively, and the columns go
+one by one through the matvec), ragged partitions, rank-0 blocks, H and H^T, both orderings and
 padded leading dimensions.
 """
 import numpy as np
