@@ -85,36 +85,46 @@ class Gmres:
         self.w = torch.zeros(self.n, dtype=dt, device=device)
         self.use_graph = use_graph
         self.graph = None
-        # CUDA: the step after the operator runs in the library's own kernels
-        # (bw_arnoldi_step, up to 4,096 steps a cycle)
-        self._work = None
-        if self.V.is_cuda and self.m <= 4096:
+        self._work = None  # scratch of bw_arnoldi_step
+        if self.V.is_cuda and self.m <= 4096 and self._on_device(0):
             self._work = torch.empty(3 * 160 * (self.m + 2), dtype=dt, device=self.V.device)
 
-    def _device_cycle(self):
-        """_cycle with each step's Gram-Schmidt in four launches."""
-        V, z, w = self.V, self.z, self.w
+    def _on_device(self, j):
+        """Whether step j takes the library's own four launches (bw_arnoldi_step)
+        after the operator, or vector operations.  The launches save latency but
+        stream the basis at a third of their rate, and every CTA adds all CTAs'
+        sums of every vector.  A step, launches / vector operations, averaged over
+        a cycle: n = 12,288, 30 steps 20 / 45 us; 98,304, 40 steps 48 / 73 us;
+        196,608, 20 steps 44 / 69 us, but 100 steps 218 / 112 us; 531,111, 30
+        steps 162 / 119 us; 20,000, 200 steps 60 / 56 us; 2,000,000, 2 steps 214 /
+        175 us.  The costs of single steps cross at j = 60 to 130 for short
+        vectors and at n (j + 1) = 3 to 8 million for long ones."""
+        return j < 64 and self.n * (j + 1) <= 5_000_000 and self.n <= 1_000_000
+
+    def _device_step(self, j, minv, zp):
+        V = self.V
         dev = V.device.index
-        step, stream = A.lib().bw_arnoldi_step, self.torch.cuda.current_stream(dev).cuda_stream
-        d = self.minv  # a plain diagonal multiplies in the step's last launch
-        fused = (isinstance(d, self.torch.Tensor) and d.dtype == V.dtype and d.device == V.device
-                 and d.shape == (self.n,) and d.is_contiguous())
-        minv, zp = (d.data_ptr(), z.data_ptr()) if fused else (0, 0)
-        for j in range(self.m):
-            if j == 0 or not fused:
-                self._precondition(V[j], z)
-            self.op(z, w)
-            A.check(step(dev, self.n, j, self.m, V.data_ptr(), self.H.data_ptr(), w.data_ptr(), minv, zp,
-                         self._work.data_ptr(), self._work.numel(), _BREAKDOWN, stream), None)
+        A.check(A.lib().bw_arnoldi_step(dev, self.n, j, self.m, V.data_ptr(), self.H.data_ptr(), self.w.data_ptr(),
+                                        minv, zp, self._work.data_ptr(), self._work.numel(), _BREAKDOWN,
+                                        self.torch.cuda.current_stream(dev).cuda_stream), None)
 
     def _cycle(self):
         """m Arnoldi steps from V[0]; fills V and H (FP64)."""
-        if self._work is not None:
-            return self._device_cycle()
         V, H, z, w = self.V, self.H, self.z, self.w
+        d = self.minv  # a plain diagonal multiplies in a device step's last launch
+        fused = (isinstance(d, self.torch.Tensor) and d.dtype == V.dtype and d.device == V.device
+                 and d.shape == (self.n,) and d.is_contiguous())
+        minv, zp = (d.data_ptr(), z.data_ptr()) if fused else (0, 0)
+        ready = False  # z holds the preconditioned V[j]
         for j in range(self.m):
-            self._precondition(V[j], z)
+            if not ready:
+                self._precondition(V[j], z)
             self.op(z, w)
+            if self._work is not None and self._on_device(j):
+                self._device_step(j, minv, zp)
+                ready = fused
+                continue
+            ready = False
             w0 = self.torch.linalg.vector_norm(w)
             Vj = V[:j + 1]
             h = Vj @ w

@@ -1,7 +1,9 @@
 """The Arnoldi step's kernels (bw_arnoldi_step) on the GPU (-m gpu) against the
 same Gmres on CPU tensors: basis, Hessenberg matrix and solutions, for vectors
 shorter than a warp, around a CTA's slice and longer than the CTAs' threads,
-the three kinds of preconditioner, and an exhausted Krylov space."""
+the three kinds of preconditioner, and an exhausted Krylov space.  Cycles that
+go over to vector operations at a later step, and no slower cycle than with
+those alone."""
 import numpy as np
 import pytest
 
@@ -28,7 +30,8 @@ def _pair(op_matrix, n, m, minv, seed):
 
 
 @pytest.mark.parametrize("kind", ["none", "vector", "callable"])
-@pytest.mark.parametrize("n,m", [(1, 1), (5, 3), (31, 8), (64, 20), (700, 33), (9473, 12), (90000, 6)])
+@pytest.mark.parametrize("n,m", [(1, 1), (5, 3), (31, 8), (64, 20), (700, 33), (9473, 12), (90000, 6), (700, 70),
+                                 (700000, 9)])
 def test_cycle_equals_the_cpu_cycle(n, m, kind):
     import torch
 
@@ -60,3 +63,28 @@ def test_exhausted_space_gives_zero_vectors():
     (Vc, Hc, xc), (Vg, Hg, xg) = _pair(d, n, 5, None, 3)
     assert float(Hg[2, 1]) == 0.0 == float(Hc[2, 1])
     assert not Vg[2:].any() and np.allclose(xg, xc, rtol=1e-12)
+
+
+@pytest.mark.parametrize("n,m", [(20000, 300), (196608, 100), (531111, 30), (2000000, 6)])
+def test_long_cycles_are_no_slower_than_vector_operations(n, m):
+    """Steps of long vectors or deep cycles: the kernels alone took 1.3 to 2.5
+    times the vector operations' time; a quarter is allowed for noise."""
+    import torch
+
+    ms = []
+    for work in (True, False):
+        d = 1.0 + torch.rand(n, dtype=torch.float64, device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+        g = Gmres(lambda x, y, d=d: torch.mul(d, x, out=y), n, m, 1.0 / d + 0.1)
+        if not work:
+            g._work = None
+        g.V[0].fill_(n ** -0.5)
+        for _ in range(3):
+            g._run_cycle()
+        ev = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+        ev[0].record()
+        for _ in range(5):
+            g._run_cycle()
+        ev[1].record()
+        torch.cuda.synchronize()
+        ms.append(ev[0].elapsed_time(ev[1]))
+    assert ms[0] <= 1.25 * ms[1], ms
