@@ -76,6 +76,7 @@ struct DevPhase {
   int64_t n_items = 0;
   int64_t n_elems = 0;
   int64_t n_gsegs = 0;
+  bool spread = false;             // long_items: the CTA-wide kernel deals them out one by one
   // Queue units [0, split.wide) run in the CTA-wide kernel, the rest in the
   // warp-per-item kernel, [split.wide, split.coop) CTA-cooperatively.
   bw::NarrowSplit split;
@@ -267,8 +268,9 @@ template <typename K> void smem_attr_once(bool (&done)[64], K kernel, int bytes)
 }
 
 template <typename S> void set_smem_attr() {
-  static bool done[64] = {};
-  smem_attr_once(done, bw::stream_panels_kernel<S>, bw::SmemLayout<S>::kTotal);
+  static bool done[2][64] = {};
+  smem_attr_once(done[0], bw::stream_panels_kernel<S, false>, bw::SmemLayout<S>::kTotal);
+  smem_attr_once(done[1], bw::stream_panels_kernel<S, true>, bw::SmemLayout<S>::kTotal);
 }
 
 int64_t align256(int64_t v) { return (v + 255) / 256 * 256; }
@@ -503,6 +505,24 @@ bw::NarrowSplit narrow_split(const bw::ChunkPlan &cp, const bw::Tuning &tune, in
   return sp;
 }
 
+// Whether three of the longest of the CTA-wide units [0, n_wide) exceed a CTA's
+// share of them.  Items are cut to a quarter or an eighth of the share, but not
+// below 8 rows, so the long stacks of a 2DS0 crack are (2DS0, BF16: 80,000
+// segments 138.8 us when the first CTAs of an early launch took three items
+// each, 112.0 with one; 300,000 segments 458 and 377; FP64 16,384 segments 66
+// and 58; on 3DR0 and 3DT0 cracks, where they are not, one item each would cost
+// up to 1%).
+bool long_items(const bw::ChunkPlan &cp, int64_t n_wide, int grid) {
+  int64_t all = 0, longest = 0;
+  for (int64_t u = 0; u < n_wide; u++) {
+    int64_t e = 0;
+    for (int32_t i = cp.item_ptr[u]; i < cp.item_ptr[u + 1]; i++) e += int64_t(cp.chunks[i].ncols) * cp.chunks[i].hpad;
+    all += e;
+    longest = std::max(longest, e);
+  }
+  return 3 * grid * longest > all;
+}
+
 // f(i, place) for every phase-2 chunk i, with a slice of the gather array for
 // each (the plan shares slices between the row parts of a panel); false when a
 // place passes the 32 bits that the exports give it.
@@ -528,6 +548,7 @@ void upload_phase(bw_hmat *h, int o, int prec, int phase) {
   dp.n_chunks = (int64_t)cp.chunks.size();
   dp.n_gsegs = (int64_t)cp.gsegs.size();
   dp.split = narrow_split(cp, h->prob.tune, h->grid);
+  dp.spread = long_items(cp, dp.split.wide, h->grid);
   if (h->plan_only) {
     auto &buf = h->host_data[o][prec][phase];
     buf.assign((size_t)ph.n_elems[prec] * es, 0);
@@ -688,7 +709,8 @@ void launch_matvec_impl(bw_hmat *h, int o, int prec, const double *x, double *y,
       a.withhold = h->take_withhold();  // the test hook applies to the CTA-wide kernel
       if (dp.split.wide > 0) {
         a.n_items = (int)dp.split.wide;
-        launch(bw::stream_panels_kernel<S>, h->grid, bw::threads_of<S>(), bw::SmemLayout<S>::kTotal, st, early, a);
+        launch(dp.spread ? bw::stream_panels_kernel<S, true> : bw::stream_panels_kernel<S, false>, h->grid,
+               bw::threads_of<S>(), bw::SmemLayout<S>::kTotal, st, early, a);
       }
       if (ev) BW_CUDA(cudaEventRecord(ev[phase == 0 ? 2 : 5], st));
       if (dp.split.wide < dp.n_items) {  // the items of at most narrow_rows rows, on their own queue

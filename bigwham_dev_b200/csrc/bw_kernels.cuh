@@ -350,20 +350,32 @@ struct ItemQueue {
       e = item_ptr[it + 1];
     }
   }
-  __device__ __forceinline__ void init(const int32_t *ptr, int n, int *q, int lane) {
+  // all: the first three items; else the first one, more() the two after it
+  __device__ __forceinline__ void init(const int32_t *ptr, int n, int *q, int lane, bool all = true) {
     item_ptr = ptr;
     n_items = n;
     queue = q;
-    int i0 = 0, i1 = 0;
+    int i0 = 0, i1 = all ? 0 : n;
     pend = n;
     if (lane == 0) {
       i0 = atomicAdd(&queue[0], 1);
-      i1 = i0 < n ? atomicAdd(&queue[0], 1) : n;
-      pend = i1 < n ? atomicAdd(&queue[0], 1) : n;
+      if (all) {
+        i1 = i0 < n ? atomicAdd(&queue[0], 1) : n;
+        pend = i1 < n ? atomicAdd(&queue[0], 1) : n;
+      }
     }
     cur = __shfl_sync(0xffffffffu, i0, 0);
     nxt = __shfl_sync(0xffffffffu, i1, 0);
     load_range(cur, cb, ce);
+    load_range(nxt, ncb, nce);
+  }
+  __device__ __forceinline__ void more(int lane) {
+    int i1 = 0;
+    if (lane == 0) {
+      i1 = cur < n_items ? atomicAdd(&queue[0], 1) : n_items;
+      pend = i1 < n_items ? atomicAdd(&queue[0], 1) : n_items;
+    }
+    nxt = __shfl_sync(0xffffffffu, i1, 0);
     load_range(nxt, ncb, nce);
   }
   __device__ __forceinline__ bool valid() const { return cur < n_items; }
@@ -406,7 +418,8 @@ template <typename S> __device__ __forceinline__ bool chunk_ok(const uint32_t (&
   return ncols > 0 && ncols <= SmemLayout<S>::kWindow && chunk_bytes_of<S>(w) <= static_cast<unsigned long long>(kStageBytes);
 }
 
-template <typename S>
+// kSpread: long items (long_items), one per CTA until all have started.
+template <typename S, bool kSpread>
 __global__ void __launch_bounds__(threads_of<S>(), 1) stream_panels_kernel(StreamArgs a) {
   using G = typename Store<S>::G;
   using L = SmemLayout<S>;
@@ -466,7 +479,13 @@ __global__ void __launch_bounds__(threads_of<S>(), 1) stream_panels_kernel(Strea
       ordered = true;
     };
     ItemQueue iq;
-    iq.init(a.item_ptr, a.n_items, a.queue, lane);
+    iq.init(a.item_ptr, a.n_items, a.queue, lane, !kSpread);
+    // CTAs may start one after the other beside the launch before.  With long
+    // items, a CTA whose first item fills the stages takes its next ones only
+    // towards that item's end, once the launch before is done and all have
+    // started: else the first CTAs take three of the longest each.
+    bool more = !kSpread || iq.ce - iq.cb <= kStages;
+    if (kSpread && more) iq.more(lane);
     // batches of up to 32 chunks of one item; lane k holds chunk k's
     // descriptor, and the next batch's descriptors load during this one
     int bb = iq.cb;
@@ -476,7 +495,7 @@ __global__ void __launch_bounds__(threads_of<S>(), 1) stream_panels_kernel(Strea
       const int be = min(bb + 32, iq.ce);
       const bool same = be < iq.ce;
       DescRegs nxt_d;
-      load_desc(a.chunks, (same ? be : iq.ncb) + lane, same ? iq.ce : iq.nce, nxt_d);
+      if (same || more) load_desc(a.chunks, (same ? be : iq.ncb) + lane, same ? iq.ce : iq.nce, nxt_d);
       {
         const int nb = be - bb;
         for (int k = 0; k < nb; k++) {
@@ -488,6 +507,11 @@ __global__ void __launch_bounds__(threads_of<S>(), 1) stream_panels_kernel(Strea
           // before the first stage is used again, and before a chunk without a
           // window (an empty one, or one refused below)
           if (!ordered && (issued == kStages || !chunk_ok<S>(w))) order();
+          if (kSpread && !more && !same && ordered) {  // the first item's last batch
+            iq.more(lane);
+            more = true;
+            load_desc(a.chunks, iq.ncb + lane, iq.nce, nxt_d);
+          }
           if (!mbar_wait(&empty[s], (use & 1u) ^ 1u, a.spin_limit)) {
             if (lane == 0) set_error(a.err, kErrTimeoutEmpty);
             ok = false;

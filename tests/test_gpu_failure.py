@@ -96,6 +96,34 @@ def test_timeout_of_several_columns(prec):
     h.close()
 
 
+@pytest.mark.parametrize("prec", ["fp64", "fp32", "bf16"])
+def test_timeout_of_long_items(prec):
+    """The same where the CTAs take their first items one by one: long items,
+    the withheld chunk in a CTA's first one (before or after it has its next)."""
+    import torch
+
+    n, k = 20_000, 200
+    rng = np.random.default_rng(0)
+    h = HmatGpu(1, 8, k * n, np.arange(8), np.arange(k * n), device=0)
+    for j in range(k):
+        h.add_lowrank(0, j * n, rng.uniform(-1, 1, (8, 1)), rng.uniform(-1, 1, (1, n)))
+    h.finalize(precisions=(prec,))
+    x = torch.from_numpy(rng.uniform(-1, 1, k * n)).cuda()
+    good = h.matvec(x, prec).clone()
+    h.sync()
+    for chunk in (0, 5, 6, 38):
+        h.set_wait_limit(20_000_000)
+        A.check(A.lib().bw_test_withhold_chunk(h._h, chunk), h._h)
+        h.matvec(x, prec)
+        with pytest.raises(BigWhamError) as e:
+            h.sync()
+        assert e.value.status == A.BW_ERR_DEVICE and "error word" in str(e.value)
+        h.set_wait_limit(2_000_000_000)
+        assert torch.equal(h.matvec(x, prec), good)
+        h.sync()
+    h.close()
+
+
 @pytest.mark.parametrize("prec", ["fp64", "fp32"])
 def test_the_limit_is_a_stage_s_not_the_launch_before_s(prec):
     """A phase-2 CTA may get its SM while phase 1 still runs elsewhere (here on
