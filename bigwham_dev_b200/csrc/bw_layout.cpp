@@ -84,9 +84,11 @@ EffLow eff_low(const Problem &p, bool tr, size_t k) {
 
 int64_t align_up(int64_t v, int64_t a) { return (v + a - 1) / a * a; }
 
-// Most entries of one item of a phase.
-int64_t item_cap(int64_t entries, int64_t grid, int items_per_cta) {
-  if (items_per_cta <= 0) items_per_cta = entries / grid < kSmallShare ? kItemsPerCtaSmall : kItemsPerCta;
+// Most entries of one item of a phase; `thinnest`: entries of the longest one that
+// cannot be cut further.
+int64_t item_cap(int64_t entries, int64_t grid, int items_per_cta, int64_t thinnest = 0) {
+  if (items_per_cta <= 0)
+    items_per_cta = entries / grid < kSmallShare || thinnest > entries / grid ? kItemsPerCtaSmall : kItemsPerCta;
   return std::max<int64_t>(1, entries / grid / items_per_cta);
 }
 
@@ -137,7 +139,9 @@ void build_operator(const Problem &p, bool tr, int grid, OperatorPlan &op) {
   grid = std::max(1, grid);
   int64_t e1 = 0;  // phase-1 entries
   for (size_t k = 0; k < nlr; k++) e1 += p.lr[k].r * eff_low(p, tr, k).n;
-  const int64_t cap1 = item_cap(e1, grid, p.tune.items_per_cta[0]);
+  int64_t widest = 0;  // columns of the longest stack
+  for (auto &kv : stacks) widest = std::max(widest, kv.first.second);
+  const int64_t cap1 = item_cap(e1, grid, p.tune.items_per_cta[0], kRowAlign * widest);
   PhasePlan &p1 = op.ph[0];
   for (auto &kv : stacks) {
     const int64_t j0 = kv.first.first, n = kv.first.second;

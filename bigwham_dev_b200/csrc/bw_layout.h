@@ -42,7 +42,10 @@ constexpr int kItemAlign = 64;       // item start alignment, in elements
 // 8 for a phase of less than kSmallShare entries per CTA, whose few items are
 // else too uneven.  Matvec at 4 / 8 items: 3DR0 FP32 3,600 DoF 44.9 / 34.9 us,
 // 27,648 DoF 111 / 125 us, 49,152 DoF 185 / 189 us (BF16 142 / 156 us), 196,608
-// DoF 888 / 888 us; 3DT0 BF16 132,150 DoF 289 / 313 us.
+// DoF 888 / 888 us; 3DT0 BF16 132,150 DoF 289 / 313 us.  8 also where the longest
+// stack, cut to kRowAlign rows, is more than a CTA's share: the others have to
+// fit around it (2DS0 FP32 45,000 segments 95.6 / 84.2 us, 60,000 116.6 / 99.8
+// us; on 2DS0 batches, whose stacks are shorter, 136.8 / 138.6 us).
 constexpr int kItemsPerCta = 4;
 constexpr int kItemsPerCtaSmall = 8;
 constexpr int64_t kSmallShare = 32768;

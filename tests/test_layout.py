@@ -133,6 +133,24 @@ def test_queue_units_group_small_items():
     assert all(np.array_equal(outs[0], o) for o in outs[1:])
 
 
+@pytest.mark.parametrize("widest,rows", [(4000, 32), (5000, 16)])
+def test_items_around_a_long_stack(widest, rows):
+    """Phase 1's stacks are cut to a quarter of a CTA's share (33,000 entries
+    here), but to an eighth where 8 rows of the longest stack exceed a share."""
+    nb, n = 122, 200
+    rng = np.random.default_rng(0)
+    h = HmatGpu(1, nb * n + 8, n + widest, np.arange(nb * n + 8), np.arange(n + widest), device=-1)
+    for k in range(nb):
+        h.add_lowrank(k * n, 0, rng.uniform(-1, 1, (n, n)), rng.uniform(-1, 1, (n, n)))
+    h.add_lowrank(nb * n, n, rng.uniform(-1, 1, (8, 1)), rng.uniform(-1, 1, (1, widest)))
+    h.add_lowrank(0, n, np.zeros((nb * n, 0)), np.zeros((0, widest)))  # the rest is zero
+    h.add_lowrank(nb * n, 0, np.zeros((8, 0)), np.zeros((0, n)))
+    h.finalize(plan_only=True)
+    p = h.plan_export("fp64", 1)
+    tall = max(decode(w)["hpad"] for w in p["chunks"])
+    assert tall == rows
+
+
 def _simple(n=8):
     return HmatGpu(1, n, n, np.arange(n), np.arange(n), device=-1)
 
