@@ -65,6 +65,12 @@ int prec_index(int flags) {
 constexpr int kTimedLaunches = 6;
 constexpr size_t kEv = kTimedLaunches + 1;
 
+// How a phase's CTA-wide units [0, n_wide) are launched.
+struct WideLaunch {
+  bool spread = false;  // the kernel deals the items out one by one
+  bool alone = false;   // no unstaged CTA beside one of this launch on its SM
+};
+
 struct DevPhase {
   void *data = nullptr;
   Chunk *chunks = nullptr;
@@ -76,7 +82,7 @@ struct DevPhase {
   int64_t n_items = 0;
   int64_t n_elems = 0;
   int64_t n_gsegs = 0;
-  bool spread = false;             // long_items: the CTA-wide kernel deals them out one by one
+  WideLaunch wide;                 // of units [0, split.wide)
   // Queue units [0, split.wide) run in the CTA-wide kernel, the rest in the
   // warp-per-item kernel, [split.wide, split.coop) CTA-cooperatively.
   bw::NarrowSplit split;
@@ -269,8 +275,8 @@ template <typename K> void smem_attr_once(bool (&done)[64], K kernel, int bytes)
 
 template <typename S> void set_smem_attr() {
   static bool done[2][64] = {};
-  smem_attr_once(done[0], bw::stream_panels_kernel<S, false>, bw::SmemLayout<S>::kTotal);
-  smem_attr_once(done[1], bw::stream_panels_kernel<S, true>, bw::SmemLayout<S>::kTotal);
+  smem_attr_once(done[0], bw::stream_panels_kernel<S, false>, bw::kSmemLimit);
+  smem_attr_once(done[1], bw::stream_panels_kernel<S, true>, bw::kSmemLimit);
 }
 
 int64_t align256(int64_t v) { return (v + 255) / 256 * 256; }
@@ -505,22 +511,36 @@ bw::NarrowSplit narrow_split(const bw::ChunkPlan &cp, const bw::Tuning &tune, in
   return sp;
 }
 
-// Whether three of the longest of the CTA-wide units [0, n_wide) exceed a CTA's
-// share of them.  Items are cut to a quarter or an eighth of the share, but not
-// below 8 rows, so the long stacks of a 2DS0 crack are (2DS0, BF16: 80,000
-// segments 138.8 us when the first CTAs of an early launch took three items
-// each, 112.0 with one; 300,000 segments 458 and 377; FP64 16,384 segments 66
-// and 58; on 3DR0 and 3DT0 cracks, where they are not, one item each would cost
-// up to 1%).
-bool long_items(const bw::ChunkPlan &cp, int64_t n_wide, int grid) {
-  int64_t all = 0, longest = 0;
-  for (int64_t u = 0; u < n_wide; u++) {
-    int64_t e = 0;
-    for (int32_t i = cp.item_ptr[u]; i < cp.item_ptr[u + 1]; i++) e += int64_t(cp.chunks[i].ncols) * cp.chunks[i].hpad;
-    all += e;
-    longest = std::max(longest, e);
+// WideLaunch::spread: three of the longest units exceed a CTA's share.  Items are cut to a
+// quarter or an eighth of the share, but not below 8 rows, so the long stacks of
+// a 2DS0 crack are (2DS0, BF16: 80,000 segments 138.8 us when the first CTAs of
+// an early launch took three items each, 112.0 with one; 300,000 segments 458
+// and 377; FP64 16,384 segments 66 and 58; on 3DR0 and 3DT0 cracks, where they
+// are not, one item each would cost up to 1%).
+// WideLaunch::alone: the phase waits for its longest unit, which takes over 0.1 ms by itself
+// and longer on a shared SM.  FP64 (the other kernels' CTAs leave no room
+// anyway), beside / alone: 65,000 segments (4.2 MB) 176.5 / 174.7 us, 70,000
+// (4.5 MB) 204 / 209, 80,000 (5.1 MB) 219 / 205, 300,000 843 / 759; three of
+// 80,000 (5.1 MB, a share of 8.5 MB) 500 / 523; 48 cracks 283 / 302.
+constexpr int64_t kAloneBytes = 4800000;
+
+WideLaunch wide_launch(const bw::ChunkPlan &cp, int64_t n_wide, int esize, int grid) {
+  int64_t wide = 0, all = 0, longest = 0;
+  const int64_t n_units = std::max<int64_t>(0, (int64_t)cp.item_ptr.size() - 1);
+  for (int64_t u = 0; u < n_units; u++) {
+    int64_t b = 0;
+    for (int32_t i = cp.item_ptr[u]; i < cp.item_ptr[u + 1]; i++)
+      b += int64_t(cp.chunks[i].ncols) * cp.chunks[i].hpad * esize;
+    all += b;
+    if (u < n_wide) {
+      wide += b;
+      longest = std::max(longest, b);
+    }
   }
-  return 3 * grid * longest > all;
+  WideLaunch w;
+  w.spread = 3 * grid * longest > wide;
+  w.alone = esize == 8 && n_wide < n_units && longest > kAloneBytes && grid * longest > all;
+  return w;
 }
 
 // f(i, place) for every phase-2 chunk i, with a slice of the gather array for
@@ -548,7 +568,7 @@ void upload_phase(bw_hmat *h, int o, int prec, int phase) {
   dp.n_chunks = (int64_t)cp.chunks.size();
   dp.n_gsegs = (int64_t)cp.gsegs.size();
   dp.split = narrow_split(cp, h->prob.tune, h->grid);
-  dp.spread = long_items(cp, dp.split.wide, h->grid);
+  dp.wide = wide_launch(cp, dp.split.wide, es, h->grid);
   if (h->plan_only) {
     auto &buf = h->host_data[o][prec][phase];
     buf.assign((size_t)ph.n_elems[prec] * es, 0);
@@ -709,8 +729,8 @@ void launch_matvec_impl(bw_hmat *h, int o, int prec, const double *x, double *y,
       a.withhold = h->take_withhold();  // the test hook applies to the CTA-wide kernel
       if (dp.split.wide > 0) {
         a.n_items = (int)dp.split.wide;
-        launch(dp.spread ? bw::stream_panels_kernel<S, true> : bw::stream_panels_kernel<S, false>, h->grid,
-               bw::threads_of<S>(), bw::SmemLayout<S>::kTotal, st, early, a);
+        launch(dp.wide.spread ? bw::stream_panels_kernel<S, true> : bw::stream_panels_kernel<S, false>, h->grid,
+               bw::threads_of<S>(), dp.wide.alone ? bw::kSmemLimit : bw::SmemLayout<S>::kTotal, st, early, a);
       }
       if (ev) BW_CUDA(cudaEventRecord(ev[phase == 0 ? 2 : 5], st));
       if (dp.split.wide < dp.n_items) {  // the items of at most narrow_rows rows, on their own queue

@@ -289,12 +289,14 @@ __device__ __forceinline__ void chunk_dot<float, 4>(const unsigned char *base, c
 }
 
 // ----------------------------------------------------------------------------- shared memory
+constexpr int kSmemLimit = 232448;  // dynamic shared memory per CTA
+
 template <typename S> struct SmemLayout {
   using G = typename Store<S>::G;
   static constexpr int kDataBytes = kStageBytes + 32;
   // vector window: the chunk's run of values with up to 15 bytes of slack each
   // side (FP64 chunks have half the columns: a phase's unstaged CTAs then fit
-  // beside this kernel's)
+  // beside this kernel's, unless the launch takes all shared memory to stay alone)
   static constexpr int kWindow = sizeof(G) == 8 ? kMaxColsFp64 : kMaxCols;
   static constexpr int kGBytes = kWindow * (int)sizeof(G) + 32;
   static constexpr int kStageSize = kDataBytes + kGBytes + (int)sizeof(Chunk);
@@ -304,7 +306,7 @@ template <typename S> struct SmemLayout {
   static constexpr int kBarBytes = (2 * kStages + 1) * 8;
   static constexpr int kTotal = kStages * kStageSize + kRedBytes + kBarBytes;
   static_assert(kStageSize % 16 == 0, "stage must keep 16-byte alignment");
-  static_assert(kTotal <= 232448, "shared memory above the 227 KB per-CTA limit");
+  static_assert(kTotal <= kSmemLimit, "shared memory above the 227 KB per-CTA limit");
 };
 
 struct DescRegs {
@@ -418,7 +420,7 @@ template <typename S> __device__ __forceinline__ bool chunk_ok(const uint32_t (&
   return ncols > 0 && ncols <= SmemLayout<S>::kWindow && chunk_bytes_of<S>(w) <= static_cast<unsigned long long>(kStageBytes);
 }
 
-// kSpread: long items (long_items), one per CTA until all have started.
+// kSpread: long items (wide_launch), one per CTA until all have started.
 template <typename S, bool kSpread>
 __global__ void __launch_bounds__(threads_of<S>(), 1) stream_panels_kernel(StreamArgs a) {
   using G = typename Store<S>::G;

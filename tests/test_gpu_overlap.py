@@ -74,6 +74,31 @@ def test_long_items_around_the_stages_and_batches(prec, tol, chunks):
         h.close()
 
 
+@pytest.mark.parametrize("n", [70_000, 80_000])
+def test_one_long_item_among_short_ones(n):
+    """FP64 phases whose longest item takes over 4.8 MB of 8 rows keep their SMs
+    to themselves (the 80,000 columns), the short items' launch after them."""
+    import torch
+
+    rng = np.random.default_rng(n)
+    k, m, r = 400, 300, 3
+    A, B = rng.uniform(-1, 1, (8, 1)), rng.uniform(-1, 1, (1, n))
+    h = HmatGpu(1, 8, n + k * m, np.arange(8), np.arange(n + k * m), device=0)
+    h.add_lowrank(0, 0, A, B)
+    short = [(rng.uniform(-1, 1, (8, r)), rng.uniform(-1, 1, (r, m))) for _ in range(k)]
+    for j, (a, b) in enumerate(short):
+        h.add_lowrank(0, n + j * m, a, b)
+    h.finalize(precisions=("fp64",))
+    p = h.plan_export("fp64", 1, with_data=False)
+    assert (p["n_wide"], len(p["item_ptr"]) - 1) == (1, 1 + k)
+    for _ in range(3):
+        x = rng.uniform(-1, 1, n + k * m)
+        y = h.matvec(torch.from_numpy(x).cuda()).cpu().numpy()
+        want = A @ (B @ x[:n]) + sum(a @ (b @ x[n + j * m:n + (j + 1) * m]) for j, (a, b) in enumerate(short))
+        assert np.linalg.norm(y - want) <= 1e-13 * np.linalg.norm(abs(A) @ (abs(B) @ abs(x[:n])))
+    h.close()
+
+
 @pytest.mark.parametrize("prec", ["fp64", "fp32", "bf16"])
 def test_long_items_go_to_ctas_of_their_own(prec):
     """One long item per CTA (148 of 20,000 columns) and a gather of 3 million
