@@ -3,10 +3,9 @@ taken term by term (end by end, corner by corner) in extended precision.
 
 The headers combine the ends and corners before they divide or take a
 logarithm or an angle; near an end or an edge, close to the element's plane
-and far away the combined forms must lose nothing.  Bars: the term-by-term
-forms in double precision stay within the same multiples of the largest value
-(near a singular line the position's own rounding, eps |x| / distance, is
-what both show).
+and far away the combined forms must lose nothing.  Bar: four times the largest
+error that the term-by-term forms show in double precision on the same points
+(over a dozen draws the ratio is at most 2.9, mostly below 1.5), or 2e-15.
 """
 import numpy as np
 import pytest
@@ -16,18 +15,18 @@ LD = np.longdouble
 PI = LD("3.14159265358979323846264338327950288")
 
 
-def s0_terms(rec, dd, pts):
-    rec, dd, pts = rec.astype(LD), dd.astype(LD), pts.astype(LD)
-    nu, g = LD(NU), LD(G)
-    c = 1 / (4 * PI * (1 - nu))
-    S, U = np.zeros((len(pts), 3), LD), np.zeros((len(pts), 2), LD)
+def s0_terms(rec, dd, pts, T=LD):
+    rec, dd, pts = rec.astype(T), dd.astype(T), pts.astype(T)
+    nu, g = T(NU), T(G)
+    c = 1 / (4 * T(PI) * (1 - nu))
+    S, U = np.zeros((len(pts), 3), T), np.zeros((len(pts), 2), T)
     for (cx, cy, a, tx, ty), (ds, dn) in zip(rec, dd.reshape(-1, 2)):
         nx, ny = -ty, tx
         dx, dy = pts[:, 0] - cx, pts[:, 1] - cy
         x, y = tx * dx + ty * dy, nx * dx + ny * dy
         xm, xp = x - a, x + a
         r1, r2 = xm * xm + y * y, xp * xp + y * y
-        ys = np.where(y == 0, LD(-0.0), y)  # on the line, from below
+        ys = np.where(y == 0, T(-0.0), y)  # on the line, from below
         fx, fy = c / 2 * (np.log(r1) - np.log(r2)), -c * (np.arctan2(ys, xm) - np.arctan2(ys, xp))
         fxy, fyy = c * (y / r1 - y / r2), -c * (xm / r1 - xp / r2)
         fxyy = c * ((xm * xm - y * y) / r1 ** 2 - (xp * xp - y * y) / r2 ** 2)
@@ -44,10 +43,10 @@ def s0_terms(rec, dd, pts):
     return S, U
 
 
-def r0_terms(rec, dd, pts):
-    rec, dd, pts = rec.astype(LD), dd.astype(LD), pts.astype(LD)
-    nu, g = LD(NU), LD(G)
-    S, U = np.zeros((len(pts), 6), LD), np.zeros((len(pts), 3), LD)
+def r0_terms(rec, dd, pts, T=LD):
+    rec, dd, pts = rec.astype(T), dd.astype(T), pts.astype(T)
+    nu, g = T(NU), T(G)
+    S, U = np.zeros((len(pts), 6), T), np.zeros((len(pts), 3), T)
     for el, (d0, d1, d2) in zip(rec, dd.reshape(-1, 3)):
         R = el[3:12].reshape(3, 3)
         x, y, z = ((pts - el[:3]) @ R.T).T
@@ -69,7 +68,7 @@ def r0_terms(rec, dd, pts):
                 for k, v in terms.items():
                     d[k] = d.get(k, 0) + s * v
         zzz = -(d["xxz"] + d["yyz"])
-        Cs, c, k1, k2 = g / (4 * PI * (1 - nu)), 1 / (8 * PI * (1 - nu)), 2 * (1 - nu), 1 - 2 * nu
+        Cs, c, k1, k2 = g / (4 * T(PI) * (1 - nu)), 1 / (8 * T(PI) * (1 - nu)), 2 * (1 - nu), 1 - 2 * nu
         xx = d0 * (2 * d["xz"] - z * d["xxx"]) + d1 * (2 * nu * d["yz"] - z * d["xxy"])
         xx = xx + d2 * (d["zz"] + k2 * d["yy"] - z * d["xxz"])
         yy = d0 * (2 * nu * d["xz"] - z * d["xyy"]) + d1 * (2 * d["yz"] - z * d["yyy"])
@@ -95,29 +94,31 @@ def _off(a, b):
     return float(np.max(np.linalg.norm(a - b, axis=1) / np.linalg.norm(b, axis=1)))
 
 
-# points around one element of half length 1 (half sides 1 and 1), and the
-# largest relative error of a point's stress and displacement vectors; the
-# term-by-term forms in double precision show 1e-14 / 5e-14 at generic points
+def _no_worse(got, terms, want):
+    """Largest relative error of a point's vector against the term-by-term form's."""
+    return _off(got, want) < max(4 * _off(terms, want), 2e-15)
+
+
+# points around one element of half length 1 (half sides 1 and 0.8)
 WHERE = {
-    "around": (lambda r, n, k: r.uniform(-2, 2, (n, k)), 1e-13),
-    "close": (lambda r, n, k: np.column_stack([r.uniform(-2, 2, (n, k - 1)),
-                                               10.0 ** r.uniform(-6, -1, n) * r.choice([-1, 1], n)]), 1e-9),
-    "end": (lambda r, n, k: np.eye(k)[0] + 1e-4 * r.standard_normal((n, k)), 1e-10),
+    "around": lambda r, n, k: r.uniform(-2, 2, (n, k)),
+    "close": lambda r, n, k: np.column_stack([r.uniform(-2, 2, (n, k - 1)),
+                                              10.0 ** r.uniform(-6, -1, n) * r.choice([-1, 1], n)]),
+    "end": lambda r, n, k: np.eye(k)[0] + 1e-4 * r.standard_normal((n, k)),
     # far away the ends and corners cancel by (size / distance)^2 or more
-    "far": (lambda r, n, k: 30.0 * r.uniform(-2, 2, (n, k)), 1e-9),
+    "far": lambda r, n, k: 30.0 * r.uniform(-2, 2, (n, k)),
 }
 
 
 @pytest.mark.parametrize("where", WHERE)
 def test_s0_combined_ends(probe, where):
-    pts, tol = WHERE[where]
-    r = np.random.default_rng(3)
-    pts = np.ascontiguousarray(pts(r, 400, 2))
+    pts = np.ascontiguousarray(WHERE[where](np.random.default_rng(3), 400, 2))
     rec, dd = np.array([[0.0, 0.0, 1.0, 1.0, 0.0]]), np.array([0.7, 1.3])
     s, u = np.empty((400, 3)), np.empty((400, 2))
     probe.probe_s0_fields(1, rec, dd, G, NU, 400, pts, s, u)
     S, U = s0_terms(rec, dd, pts)
-    assert _off(s, S) < tol and _off(u, U) < tol
+    Sd, Ud = s0_terms(rec, dd, pts, np.float64)
+    assert _no_worse(s, Sd, S) and _no_worse(u, Ud, U)
 
 
 @pytest.mark.parametrize("x", [0.3, -0.7, 1.5, -2.0])
@@ -132,12 +133,11 @@ def test_s0_on_the_line(probe, x):
 
 @pytest.mark.parametrize("where", WHERE)
 def test_r0_combined_corners(probe, where):
-    pts, tol = WHERE[where]
-    r = np.random.default_rng(4)
-    pts = np.ascontiguousarray(pts(r, 400, 3))
+    pts = np.ascontiguousarray(WHERE[where](np.random.default_rng(4), 400, 3))
     rec = np.hstack([np.zeros(3), np.eye(3).ravel(), [0, 0, 1.0], [1.0, 0.8]])[None, :].copy()
     dd = np.array([0.7, -0.4, 1.3])
     s, u = np.empty((400, 6)), np.empty((400, 3))
     probe.probe_r0_fields(1, rec, dd, G, NU, 400, pts, s, u)
     S, U = r0_terms(rec, dd, pts)
-    assert _off(s, S) < 10 * tol and _off(u, U) < 10 * tol
+    Sd, Ud = r0_terms(rec, dd, pts, np.float64)
+    assert _no_worse(s, Sd, S) and _no_worse(u, Ud, U)

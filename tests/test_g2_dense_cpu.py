@@ -1,5 +1,5 @@
 """gather_g2_kernel's dealing of run values to lanes, restated in numpy: each
-warp takes 32 runs (lane k: run k, zero length past the end), an inclusive
+warp takes 2 to 32 runs (lane k: run k, zero length past them), an inclusive
 scan gives every run its first position in the warp's value list, and each
 round of 32 positions [w0, w0 + 32) finds the run of w0 + j as the last run
 starting at or before w0 (a ballot) plus the number of run starts inside
@@ -11,21 +11,22 @@ may be skipped but nothing is read or written outside a run.
 """
 import numpy as np
 import pytest
-from planreplay import build_g2, gather_runs
+from planreplay import build_g2, slices
 
 from bigwham_dev_b200 import HmatGpu
 
-KG2RUNS, UNROLL = 32, 4
+UNROLL = 4
+PER_WARP = [2, 4, 8, 16, 32]  # g2_runs_per_warp
 
 
-def dense_g2(runs, x, t, n):
+def dense_g2(runs, x, t, n, per_warp):
     """Lane-level restatement of gather_g2_kernel over all warps; returns G2,
     the write count per entry and the (source flag, index) of every read."""
     g2 = np.zeros(n)
     written = np.zeros(n, dtype=np.int64)
     reads = []
-    for r0 in range(0, len(runs), KG2RUNS):
-        w = runs[r0:r0 + KG2RUNS]
+    for r0 in range(0, len(runs), per_warp):
+        w = runs[r0:r0 + per_warp]
         cols = np.zeros(32, dtype=np.int64)
         dst = np.zeros(32, dtype=np.int64)
         off = np.zeros(32, dtype=np.int64)
@@ -59,11 +60,11 @@ def dense_g2(runs, x, t, n):
     return g2, written, reads
 
 
-def _check(runs, x, t):
+def _check(runs, x, t, per_warp):
     cols = (runs[:, 2].view(np.uint32) & 0x7FFFFFFF).astype(np.int64)
     assert np.all(cols > 0)  # the layout makes no empty run
     want = build_g2(runs, x, t)
-    got, written, _ = dense_g2(runs, x, t, want.size)
+    got, written, _ = dense_g2(runs, x, t, want.size, per_warp)
     covered = np.zeros(want.size, dtype=np.int64)
     for d, c in zip(runs[:, 0].astype(np.int64), cols):
         covered[d:d + c] += 1
@@ -82,8 +83,9 @@ def _runs(cols, rng, n_src=5000):
     return runs
 
 
+@pytest.mark.parametrize("per_warp", PER_WARP)
 @pytest.mark.parametrize("precision", ["fp32", "bf16"])
-def test_dense_g2_on_synthetic_partitions(precision):
+def test_dense_g2_on_synthetic_partitions(precision, per_warp):
     from synth import synthetic_hmat
 
     for npr, npc, dof, leaf in [(300, 300, 2, 20), (600, 600, 2, 32), (17, 60, 3, 8)]:
@@ -94,19 +96,21 @@ def test_dense_g2_on_synthetic_partitions(precision):
         x = rng.uniform(-1, 1, arr.n_cols)
         t = rng.uniform(-1, 1, max(1, h.info()["sum_rank"]))
         for tr in (False, True):
-            _check(gather_runs(h, precision, tr), x if not tr else rng.uniform(-1, 1, arr.n_rows), t)
+            _check(slices(h, precision, tr)[2], x if not tr else rng.uniform(-1, 1, arr.n_rows), t, per_warp)
 
 
-def test_dense_g2_on_hand_made_runs():
+@pytest.mark.parametrize("per_warp", PER_WARP)
+def test_dense_g2_on_hand_made_runs(per_warp):
     """Runs of 1 to 99 values, runs longer than a round, a partial last warp."""
     rng = np.random.default_rng(5)
     cols = rng.integers(1, 40, 75)
     cols[[3, 40]] = [97, 99]
     x, t = rng.uniform(-1, 1, 5000), rng.uniform(-1, 1, 5000)
-    _check(_runs(cols, rng), x, t)
+    _check(_runs(cols, rng), x, t, per_warp)
 
 
-def test_dense_g2_with_empty_runs_stays_inside_the_runs():
+@pytest.mark.parametrize("per_warp", PER_WARP)
+def test_dense_g2_with_empty_runs_stays_inside_the_runs(per_warp):
     """Empty runs (no layout makes them) may cost values, but every read and
     write stays inside some run."""
     rng = np.random.default_rng(6)
@@ -115,7 +119,7 @@ def test_dense_g2_with_empty_runs_stays_inside_the_runs():
     runs = _runs(cols, rng)
     x, t = rng.uniform(-1, 1, 5000), rng.uniform(-1, 1, 5000)
     n = int((runs[:, 0] + cols).max())
-    _, written, reads = dense_g2(runs, x, t, n)
+    _, written, reads = dense_g2(runs, x, t, n, per_warp)
     assert written.max() <= 1
     src = (runs[:, 2].view(np.uint32) >> 31).astype(np.int64)
     for s_flag, i, d in reads:

@@ -3,14 +3,16 @@ in numpy over an exported host plan: the same descriptor words, the same
 element indices (column slots of 16-byte row runs for FP64 / FP32, (column,
 row-group, column-group) lanes over 8x8 tiles for BF16), the same reductions
 over a warp's column lanes and, for CTA-cooperative units (an item's chunks
-dealt round robin to 16 warps), over the warps.
+dealt round robin to 16 warps) and teams of 2 to 16 warps (each chunk's columns
+dealt to the team), over the warps.
 
 Each phase's queue units divide at bw_plan_split: units before n_wide run in
 the CTA-wide kernel (restated by planreplay.run_phase), [n_wide, n_coop) a
-CTA per unit and the rest warp per unit.  The split is checked against its
-rule (by default n_wide = n_coop = one past the last unit with an item of
-more than 64 padded rows or 512 columns; with narrow_coop 1, n_wide stops at
-the last tall unit and n_coop at the last long one), and the replay of both
+CTA per unit and the rest warp or team per unit.  The split is checked against
+its rule (by default n_wide = n_coop = one past the last unit with an item of
+more than 64 padded rows or 512 columns, or all units where those are a CTA
+each and the rest at most a quarter of them; with narrow_coop 1, n_wide stops
+at the last tall unit and n_coop at the last long one), and the replay of both
 launches against the oracle on the golden cases and on synthetic partitions,
 H and H^T, every precision within its rounding bound.
 """
@@ -22,11 +24,21 @@ from bigwham_dev_b200 import HmatGpu
 from oracle import oracle_matvec_perm, oracle_rmatvec_perm
 
 NARROW_ROWS, NARROW_COLS = 64, 512
+CTAS = 148
 TOL = {"fp64": 1e-13, "fp32": 2e-6, "bf16": 1e-2}
 
 
-def _lanes_fp(hpad, ncols, R):
-    """(lane, first row, columns) of a warp over a column-major chunk."""
+def narrow_team(units):
+    """Warps per unit: the most that leave every unit a team of its own among
+    two CTAs of 16 warps per SM."""
+    team = 16
+    while team > 1 and units * team > 2 * CTAS * 16:
+        team //= 2
+    return team
+
+
+def _lanes_fp(hpad, ncols, R, tw, team):
+    """(lane, first row, columns) of warp tw of a team over a column-major chunk."""
     lpc = 1
     while lpc * R < hpad:
         lpc *= 2
@@ -34,12 +46,12 @@ def _lanes_fp(hpad, ncols, R):
     for lane in range(32):
         r0 = (lane % lpc) * R
         if r0 < hpad:
-            yield lane, r0, range(lane // lpc, ncols, cpp)
+            yield lane, r0, range(lane // lpc + cpp * tw, ncols, cpp * team)
 
 
-def _lanes_bf16(hpad, ncols):
-    """(lane, column group, column, row groups) of a warp over an 8x8-tiled
-    chunk."""
+def _lanes_bf16(hpad, ncols, tw, team):
+    """(lane, column group, column, row groups) of warp tw of a team over an
+    8x8-tiled chunk."""
     nrg = hpad // 8
     rgl = 1 if nrg <= 1 else 2 if nrg <= 2 else 4
     gpw = 4 // rgl
@@ -47,33 +59,34 @@ def _lanes_bf16(hpad, ncols):
     for lane in range(32):
         c8, rl, cs = lane & 7, (lane >> 3) % rgl, (lane >> 3) // rgl
         rgs = [g for g in (rl, rl + 4) if g < nrg and (g == rl or nrg > 4)]
-        for cg in range(cs, ncg, gpw):
+        for cg in range(cs + gpw * tw, ncg, gpw * team):
             c = 8 * cg + c8
             if c < ncols:
                 yield lane, cg, c, rgs
 
 
-def _warp_chunk(plan, gsrc, precision, d, acc):
-    """One warp's pass over one chunk: acc[lane, row] += the lane's products."""
+def _warp_chunk(plan, gsrc, precision, d, acc, tw=0, team=1):
+    """Warp tw of a team over one chunk: acc[lane, row] += the lane's products."""
     data = plan["data"]
     hpad, ncols, off, g = d["hpad"], d["ncols"], d["data_off"], d["g_off"]
     assert 0 < hpad <= NARROW_ROWS and hpad % 8 == 0
     if precision == "bf16":
-        for lane, cg, c, rgs in _lanes_bf16(hpad, ncols):
+        for lane, cg, c, rgs in _lanes_bf16(hpad, ncols, tw, team):
             for rg in rgs:
                 e = off + cg * 8 * hpad + rg * 64 + (c & 7) * 8
                 acc[lane, rg * 8:rg * 8 + 8] += data[e:e + 8] * gsrc[g + c]
     else:
         R = {"fp64": 2, "fp32": 4}[precision]
-        for lane, r0, cols in _lanes_fp(hpad, ncols, R):
+        for lane, r0, cols in _lanes_fp(hpad, ncols, R, tw, team):
             for c in cols:
                 e = off + c * hpad + r0
                 acc[lane, r0:r0 + R] += data[e:e + R] * gsrc[g + c]
 
 
-def narrow_unit(plan, gsrc, out, precision, cb, ce, cta):
-    """One queue unit, warp per unit (cta False) or CTA per unit: warp w of 16
-    takes the item's chunks w, w + 16, ..., the warps' rows summed at the end."""
+def narrow_unit(plan, gsrc, out, precision, cb, ce, cta, team=1):
+    """One queue unit: a team per unit, whose warps share every chunk's columns,
+    or (cta) a CTA per unit: warp w of 16 takes the item's chunks w, w + 16, ...;
+    the warps' rows are summed at the end."""
     ds = [decode(plan["chunks"][i]) for i in range(cb, ce)]
     items, start = [], 0
     for k, d in enumerate(ds):
@@ -84,10 +97,13 @@ def narrow_unit(plan, gsrc, out, precision, cb, ce, cta):
     for item in items:
         assert item[0]["flags"] & 1
         last = item[-1]
-        nw = 16 if cta else 1
+        nw = 16 if cta else team
         acc = np.zeros((nw, 32, last["hpad"]))  # per warp, per lane, per item row
         for k, d in enumerate(item):
-            _warp_chunk(plan, gsrc, precision, d, acc[k % nw])
+            if cta:
+                _warp_chunk(plan, gsrc, precision, d, acc[k % nw])
+            for tw in range(0 if cta else team):
+                _warp_chunk(plan, gsrc, precision, d, acc[tw], tw, team)
         rows = acc.sum(axis=1).sum(axis=0)[:last["rows"]]  # lanes by shuffles, then warps in order
         out[last["out_off"]:last["out_off"] + last["rows"]] = rows
     return out
@@ -105,28 +121,32 @@ def split_rule(plan, rows=NARROW_ROWS, coop=0):
             last_long = u if cols > NARROW_COLS else last_long
     if coop:
         return last_tall + 1, max(last_tall + 1, last_long + 1)
-    return max(last_tall, last_long) + 1, max(last_tall, last_long) + 1
+    wide, n = max(last_tall, last_long) + 1, len(units) - 1
+    if wide >= CTAS and 4 * (n - wide) <= wide:
+        wide = n
+    return wide, wide
 
 
-def split_phase(plan, gsrc, out, precision, rows=NARROW_ROWS, coop=0):
+def split_phase(plan, gsrc, out, precision, rows=NARROW_ROWS, coop=0, team=None):
     n_wide, n_coop = plan["n_wide"], plan["n_coop"]
     assert (n_wide, n_coop) == split_rule(plan, rows, coop)
     wide = dict(plan, item_ptr=plan["item_ptr"][:n_wide + 1])
     run_phase(wide, gsrc, out, precision == "bf16")
     units = plan["item_ptr"]
+    team = team or narrow_team(len(units) - 1 - n_coop)
     for u in range(n_wide, len(units) - 1):
-        narrow_unit(plan, gsrc, out, precision, units[u], units[u + 1], u < n_coop)
+        narrow_unit(plan, gsrc, out, precision, units[u], units[u + 1], u < n_coop, team)
     return n_wide, n_coop, len(units) - 1
 
 
-def narrow_replay(h, x_perm, precision, transposed=False, rows=NARROW_ROWS, coop=0):
+def narrow_replay(h, x_perm, precision, transposed=False, rows=NARROW_ROWS, coop=0, team=None):
     p1 = h.plan_export(precision, 1, transposed)
     p2, runs, _ = device_phase2(h, precision, transposed)
     t = np.zeros(max(1, h.info()["sum_rank"]))
-    s1 = split_phase(p1, x_perm, t, precision, rows, coop)
+    s1 = split_phase(p1, x_perm, t, precision, rows, coop, team)
     g2 = build_g2(runs, x_perm, t)
     y = np.full(h.n_cols if transposed else h.n_rows, np.nan)
-    s2 = split_phase(p2, g2, y, precision, rows, coop)
+    s2 = split_phase(p2, g2, y, precision, rows, coop, team)
     return y, (s1, s2)
 
 
@@ -190,6 +210,43 @@ def test_split_restatement_on_synthetic_partitions(npr, npc, dof, leaf, precisio
     g = np.random.default_rng(4).uniform(-1, 1, arr.n_rows)
     yt, _ = narrow_replay(h, g, precision, transposed=True, rows=rows, coop=coop)
     assert _rel(yt, oracle_rmatvec_perm(arr, g, 1)) < TOL[precision]
+
+
+@pytest.mark.parametrize("team", [1, 2, 4, 8, 16])
+@pytest.mark.parametrize("precision", ["fp64", "fp32", "bf16"])
+def test_every_team_size(precision, team):
+    """The unstaged kernel's answer with each number of warps per unit (the
+    kernel's own follows narrow_team: 16 for these few units)."""
+    from synth import synthetic_hmat
+
+    for npr, npc, dof, leaf in [(40, 25, 2, 4), (90, 70, 3, 32), (200, 130, 1, 32)]:
+        arr = synthetic_hmat(npr, npc, dof, seed=npr + npc + leaf, leaf=leaf, rank0_share=0.2)
+        h = HmatGpu.from_flat(arr.dof, arr.n_rows, arr.n_cols, arr.fr, arr.lr, arr.fr_data, arr.lr_data, arr.perm0,
+                              arr.perm1, device=-1, plan_only=True, precisions=(precision,))
+        x = np.random.default_rng(3).uniform(-1, 1, arr.n_cols)
+        y, _ = narrow_replay(h, x, precision, team=team)
+        assert _rel(y, oracle_matvec_perm(arr, x, 1)) < TOL[precision]
+
+
+def test_a_few_units_left_over_run_cta_wide():
+    """With a unit for every CTA in the CTA-wide launch, at most a quarter as
+    many unstaged ones go there too; more stay unstaged (split_rule)."""
+    seen = set()
+    for short in (20, 200):  # panels of 8 rows beside the 200 of 72
+        rng = np.random.default_rng(short)
+        tall, rows, cols = 200, 72, 40
+        n = tall * rows + short * 8
+        h = HmatGpu(1, n, cols, np.arange(n), np.arange(cols), device=-1)
+        h.set_tuning(items_per_cta_phase2=1)
+        for k in range(tall):
+            h.add_full(k * rows, 0, rng.uniform(-1, 1, (rows, cols)))
+        for k in range(short):
+            h.add_full(tall * rows + 8 * k, 0, rng.uniform(-1, 1, (8, cols)))
+        h.finalize(plan_only=True)
+        p = h.plan_export("fp64", 2, with_data=False)
+        assert (p["n_wide"], p["n_coop"]) == split_rule(p)
+        seen.add((len(p["item_ptr"]) - 1, p["n_wide"]))
+    assert seen == {(220, 220), (400, 200)}
 
 
 def test_launch_count_follows_the_split():
