@@ -1872,7 +1872,9 @@ int fields_entry(const char *name, int device, int64_t n_elems, const double *re
     if (!(G > 0.0) || !(nu > -1.0 && nu < 0.5)) throw std::invalid_argument(std::string(name) + ": bad G or nu");
     if (n_pts == 0) return BW_OK;
     BW_CUDA(cudaSetDevice(device));
-    const int lanes = bw::field_lanes(n_pts), per_cta = bw::kFieldThreads / lanes;
+    int sms = 0;
+    BW_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    const int lanes = bw::field_lanes(n_pts, sms), per_cta = bw::kFieldThreads / lanes;
     launch(static_cast<int>(std::min<int64_t>((n_pts + per_cta - 1) / per_cta, int64_t(1) << 30)), lanes);
     BW_CUDA(cudaGetLastError());
     return BW_OK;
@@ -2199,12 +2201,14 @@ int bw_r0_aca(int device, int64_t n_elems, const double *records, double G, doub
                    order.begin();
       slots[c] = c == 0 ? slot : 11 * bw::kAcaSide[2 - c] + 2;
     }
+    BW_CUDA(cudaSetDevice(device));
+    int sms = 0;
+    BW_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     for (int c = 0; c < 3; c++) {
-      ctas[c] = (int)std::min<int64_t>(first[c + 1] - first[c], 148 * (bw::kAcaResident / threads[c]));
+      ctas[c] = (int)std::min<int64_t>(first[c + 1] - first[c], sms * (bw::kAcaResident / threads[c]));
       scratch_at[c + 1] = scratch_at[c] + slots[c] * ctas[c];
     }
     order.insert(order.end(), 3, 0);
-    BW_CUDA(cudaSetDevice(device));
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     // one device allocation for the call's tables, scratch and results
     const int64_t parts[7] = {8 * (int64_t)bw::r0::kFrameDoubles * n_elems, 4 * (int64_t)p32.size(),

@@ -4,7 +4,7 @@
 // of the element's field times its local DD (bw_s0.h, bw_r0_fields.h).
 //
 // Both kernels are bound by FP64 arithmetic: per (point, element) pair one or
-// two logs and atan2, one to five divisions and 100 to 400 other operations,
+// two logs and atan2, one (2DS0) or six (3DR0) divisions and 100 to 400 other operations,
 // against 9 or 17 doubles of element data that a tile in shared memory gives
 // to all points of the CTA.  What a pair needs is in the element headers; what
 // is left is to keep the FP64 pipe busy:
@@ -30,11 +30,11 @@ constexpr int kFieldTile = 128;     // elements per shared-memory tile
 // two threads for each of 1,024 per SM.  2DS0, 4,000 segments: 50,000 points
 // 8.05 -> 2.46 ms with the element's combined forms, 300 to 1,000 points up to
 // 60 times faster; 3DR0, 4,096 elements, 20,000 points 36.0 -> 4.52 ms.
-constexpr long long kFieldThreadsWanted = 2LL * 148 * 1024;
+constexpr long long kFieldThreadsWanted = 2 * 1024;  // per SM
 
-inline int field_lanes(long long n_pts) {
+inline int field_lanes(long long n_pts, int sms) {
   int lanes = 1;
-  while (lanes < 32 && n_pts * lanes < kFieldThreadsWanted) lanes <<= 1;
+  while (lanes < 32 && n_pts * lanes < kFieldThreadsWanted * sms) lanes <<= 1;
   return lanes;
 }
 

@@ -87,7 +87,8 @@ class Gmres:
         self.graph = None
         self._work = None  # scratch of bw_arnoldi_step
         if self.V.is_cuda and self.m <= 4096 and self._on_device(0):
-            self._work = torch.empty(3 * 160 * (self.m + 2), dtype=dt, device=self.V.device)
+            sms = torch.cuda.get_device_properties(self.V.device).multi_processor_count
+            self._work = torch.empty(3 * sms * (self.m + 2), dtype=dt, device=self.V.device)
 
     def _on_device(self, j):
         """Whether step j takes the library's own four launches (bw_arnoldi_step)
