@@ -18,7 +18,8 @@
 // block took most of the time before), and the blocks come from a queue,
 // longest first, so that the largest does not start last.
 // A 64 x 64 crack's 1,584 blocks, one call of bw_r0_aca: 18.5 ms at first, 6.1 ms
-// with this pass, the queue and a launch per size (kAcaSide).
+// with this pass, the queue and a launch per size (kAcaSide).  The three sizes are
+// held to 128 registers and spill 224 to 312 bytes of the off-plane entry.
 // Every stop decision is taken from values in shared memory that all threads
 // read, so all threads leave the loop together.  Factor storage per block is
 // capacity-bounded (cap blocks of rank); a block that needs more reports

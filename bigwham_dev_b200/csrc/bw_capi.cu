@@ -681,9 +681,15 @@ void launch_matvec_impl(bw_hmat *h, int o, int prec, const double *x, double *y,
   G *t = static_cast<G *>(t_buf);
   if (ev) BW_CUDA(cudaEventRecord(ev[0], st));
   // Each launch but the first may start while the one before it runs (not
-  // with timing events between them).  A kernel lets its successor start only
-  // after its own wait, so no more than two neighbours overlap, and the first
-  // launch of the next matvec comes after everything here.  12,288 DoF FP64
+  // with timing events between them).  The gathers and the CTA-wide launches let
+  // their successor start only after their own wait (the x gather, an ordinary
+  // launch, at once); a phase's unstaged launch does so at its start, so the
+  // CTA-wide launch before it, itself and the one after it may be resident
+  // together.  What holds: every launch reads its vector only after the wait that
+  // follows the vector's writer (an unstaged second launch starts after its
+  // CTA-wide one has waited), and every launch ends with or after its wait, so
+  // they complete in order and the first launch of the next matvec comes after
+  // everything here.  12,288 DoF FP64
   // 85.8 -> 75.7 us, a 256-segment crack 20.4 -> 17.0 us, 16,384 segments BF16
   // 54.8 -> 37.4 us.
   const bool early = !ev;
@@ -838,7 +844,8 @@ void launch_matmat_tc(bw_hmat *h, int o, const double *X, int64_t ldx, double *Y
 
 // Scratch and run tables of the FP64 / FP32 products with several right-hand
 // sides (bw_multi_kernels.cuh): 8 columns of x and t and 8 bytes per phase-2
-// chunk, about 1% of the block data, in one allocation.  Taken last; when it
+// chunk, 0.9% (3DT0) to 2.4% (3DR0) and 4.7% (2DS0) of the block data, in one
+// allocation with every FP64 / FP32 handle.  Taken last; when it
 // does not fit (the device limit, or the device itself) such products apply
 // one matvec per column, as they do without these kernels.
 void alloc_multi(bw_hmat *h, int mask, bool with_t) {

@@ -493,7 +493,9 @@ void build_chunks(const Problem &p, bool tr, int prec, int grid, OperatorPlan &o
     // Queue units: runs of consecutive items, closed once their cost
     // reaches unit_bytes (a large item is a unit by itself).  The kernel
     // walks a unit's chunks as one range; item boundaries stay in the chunk
-    // flags, so results do not depend on the grouping.
+    // flags, so the grouping does not change the results of the CTA-wide kernel
+    // (in the unstaged one the number of units sets the team, narrow_team, and
+    // with it the order of additions).
     cp.chunks.clear();
     cp.ranges.clear();
     cp.item_ptr.assign(1, 0);

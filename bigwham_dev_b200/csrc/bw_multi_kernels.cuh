@@ -14,12 +14,13 @@
 // stage.  A G2 of K columns would be written and read once more per pass: on a
 // 27,648-DoF 3DR0 crack 97 MB on top of 530 MB of FP32 blocks.
 //
-// What bounds it: the block data, as in the matvec.  Per staged 16 bytes a
-// thread reads K values of the vector window (broadcasts) and issues 4 K (FP32)
-// or 2 K (FP64) FMAs; at 44 bytes/ns per SM, K = 8 keeps the FMA pipes about a
-// third busy, so the pass costs what one matvec costs.  K = 16 would take twice
-// the registers and stage room and be bound by the FMAs.  Four stages of 48 KB
-// (K = 8) fit beside one reduction buffer.
+// What bounds it: shared memory and the per-chunk round trip.  Per staged 16
+// bytes a thread reads K values of the vector window (broadcasts within a column
+// group, bank conflicts between groups) and issues 4 K (FP32) or 2 K (FP64) FMAs,
+// which keep the FMA pipes about a third busy.  A pass of 8 columns costs 1.5 to
+// 1.7 matvecs (3DR0 FP32, 27,648 DoF: 176 us, the matvec 111, the block data 83).
+// K = 16 would take twice the registers and stage room and be bound by the FMAs.
+// Four stages of 48 KB (K = 8) fit beside one reduction buffer.
 #pragma once
 
 #include "bw_kernels.cuh"

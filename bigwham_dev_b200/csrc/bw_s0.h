@@ -48,8 +48,11 @@ constexpr double kPi = 3.14159265358979323846;
 // |zeta|^2 = r1^2 r2^2, whose parts are the second and third derivatives; the
 // two logarithms are one of the ratio and the two angles one, the angle the
 // segment subtends.  A pair costs one division, one log and one atan2 (eight
-// divisions and two of each when every term is taken by itself), and the far
-// field loses no digits to the difference of two nearly equal ends.
+// divisions and two of each when every term is taken by itself), and the
+// derivatives lose no digits to the difference of two nearly equal ends in the
+// far field.  f_x does: the logarithm of a ratio near 1 has an error of eps x
+// distance / length (3e-15 at 100 half lengths, a tenth of the term-by-term
+// form's).
 struct Derivs {
   double fx, fy, fxy, fyy, fxyy, fyyy;
 };
