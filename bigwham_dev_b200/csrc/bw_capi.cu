@@ -518,8 +518,8 @@ bw::NarrowSplit narrow_split(const bw::ChunkPlan &cp, const bw::Tuning &tune, in
 // and 377; FP64 16,384 segments 66 and 58; on 3DR0 and 3DT0 cracks, where they
 // are not, one item each would cost up to 1%).
 // WideLaunch::alone: the phase waits for its longest unit, which takes over 0.1 ms by itself
-// and longer on a shared SM.  FP64 (the other kernels' CTAs leave no room
-// anyway), beside / alone: 65,000 segments (4.2 MB) 176.5 / 174.7 us, 70,000
+// and longer on a shared SM.  FP64 only (FP32 no difference, BF16 CTAs leave no
+// room), beside / alone: 65,000 segments (4.2 MB) 176.5 / 174.7 us, 70,000
 // (4.5 MB) 204 / 209, 80,000 (5.1 MB) 219 / 205, 300,000 843 / 759; three of
 // 80,000 (5.1 MB, a share of 8.5 MB) 500 / 523; 48 cracks 283 / 302.
 constexpr int64_t kAloneBytes = 4800000;
