@@ -128,3 +128,32 @@ def test_long_items_go_to_ctas_of_their_own(prec):
     ms, count = h.timing_read_launches()
     assert count == 20 and ev[0].elapsed_time(ev[1]) < sum(ms)
     h.close()
+
+
+def test_64_columns_deal_their_items_evenly():
+    """The tensor-core product's phase 1, whose CTAs also start one after the
+    other beside the gather of X: an item per CTA takes half the time of two
+    (0.185 and 0.365 ms; 0.213 and 0.359 when the first CTAs took three each)."""
+    import torch
+
+    ms = []
+    for k in (148, 296):
+        n = 8_000
+        rng = np.random.default_rng(0)
+        h = HmatGpu(1, 8, k * n, np.arange(8), np.arange(k * n), device=0)
+        for j in range(k):
+            h.add_lowrank(0, j * n, rng.uniform(-1, 1, (8, 1)), rng.uniform(-1, 1, (1, n)))
+        h.finalize(precisions=("bf16",), matmat=True)
+        X = torch.from_numpy(rng.uniform(-1, 1, (64, k * n))).cuda().t()
+        Y = torch.empty((64, 8), dtype=torch.float64, device="cuda").t()
+        for _ in range(3):
+            h.matmat(X, "bf16", out=Y)
+        ev = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+        ev[0].record()
+        for _ in range(10):
+            h.matmat(X, "bf16", out=Y)
+        ev[1].record()
+        h.sync()
+        ms.append(ev[0].elapsed_time(ev[1]) / 10)
+        h.close()
+    assert ms[1] > 1.8 * ms[0]
