@@ -511,12 +511,15 @@ bw::NarrowSplit narrow_split(const bw::ChunkPlan &cp, const bw::Tuning &tune, in
   return sp;
 }
 
-// WideLaunch::spread: three of the longest units exceed a CTA's share.  Items are cut to a
-// quarter or an eighth of the share, but not below 8 rows, so the long stacks of
-// a 2DS0 crack are (2DS0, BF16: 80,000 segments 138.8 us when the first CTAs of
+// WideLaunch::spread: the longest unit is over two thirds of a CTA's share, so that
+// three are twice the share, and has more chunks than stages (else its CTA needs
+// its next ones at once).  Items are cut to a quarter or an eighth of the share,
+// but not below 8 rows, so the long stacks of a 2DS0 crack are, and the panels
+// of small 3DR0 ones (2DS0, BF16: 80,000 segments 138.8 us when the first CTAs of
 // an early launch took three items each, 112.0 with one; 300,000 segments 458
-// and 377; FP64 16,384 segments 66 and 58; on 3DR0 and 3DT0 cracks, where they
-// are not, one item each would cost up to 1%).
+// and 377; FP64 16,384 segments 66 and 58; 3DR0 FP64 5,043 DoF, 0.9 of a share,
+// 48.9 and 45.4; 9,408 DoF, 0.45, 59.8 and 60.8; FP32 6,075 DoF, 6 chunks, 34.1
+// and 35.1; on large 3DR0 and 3DT0 cracks one item each would cost up to 1%).
 // WideLaunch::alone: the phase waits for its longest unit, which takes over 0.1 ms by itself
 // and longer on a shared SM.  FP64 only (FP32 no difference, BF16 CTAs leave no
 // room), beside / alone: 65,000 segments (4.2 MB) 176.5 / 174.7 us, 70,000
@@ -526,6 +529,7 @@ constexpr int64_t kAloneBytes = 4800000;
 
 WideLaunch wide_launch(const bw::ChunkPlan &cp, int64_t n_wide, int esize, int grid) {
   int64_t wide = 0, all = 0, longest = 0;
+  int32_t chunks = 0;  // of the longest
   const int64_t n_units = std::max<int64_t>(0, (int64_t)cp.item_ptr.size() - 1);
   for (int64_t u = 0; u < n_units; u++) {
     int64_t b = 0;
@@ -534,11 +538,14 @@ WideLaunch wide_launch(const bw::ChunkPlan &cp, int64_t n_wide, int esize, int g
     all += b;
     if (u < n_wide) {
       wide += b;
-      longest = std::max(longest, b);
+      if (b > longest) {
+        longest = b;
+        chunks = cp.item_ptr[u + 1] - cp.item_ptr[u];
+      }
     }
   }
   WideLaunch w;
-  w.spread = 3 * grid * longest > wide;
+  w.spread = 3 * grid * longest > 2 * wide && chunks > bw::kStages;
   w.alone = esize == 8 && n_wide < n_units && longest > kAloneBytes && grid * longest > all;
   return w;
 }

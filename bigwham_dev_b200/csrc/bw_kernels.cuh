@@ -420,7 +420,7 @@ template <typename S> __device__ __forceinline__ bool chunk_ok(const uint32_t (&
   return ncols > 0 && ncols <= SmemLayout<S>::kWindow && chunk_bytes_of<S>(w) <= static_cast<unsigned long long>(kStageBytes);
 }
 
-// kSpread: long items (wide_launch), one per CTA until all have started.
+// kSpread: long items (WideLaunch), one per CTA until all have started.
 template <typename S, bool kSpread>
 __global__ void __launch_bounds__(threads_of<S>(), 1) stream_panels_kernel(StreamArgs a) {
   using G = typename Store<S>::G;
