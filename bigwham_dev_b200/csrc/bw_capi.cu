@@ -259,24 +259,24 @@ template <typename F> int guarded(bw_hmat *h, F &&f) {
   }
 }
 
-// Dynamic shared-memory opt-in of a kernel, set once per device.  The flags
+// Dynamic shared-memory opt-in of kernels, set once per device.  The flags
 // are guarded by one mutex: first calls from several host threads (one per
 // device, or several handles on one device) do not race on them.
 std::mutex g_attr_mu;
 
-template <typename K> void smem_attr_once(bool (&done)[64], K kernel, int bytes) {
+template <typename... K> void smem_attr_once(bool (&done)[64], int bytes, K... kernels) {
   int dev = 0;
   BW_CUDA(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> g(g_attr_mu);
   if (dev < 64 && done[dev]) return;
-  BW_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  for (const void *k : {reinterpret_cast<const void *>(kernels)...})
+    BW_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
   if (dev < 64) done[dev] = true;
 }
 
 template <typename S> void set_smem_attr() {
-  static bool done[2][64] = {};
-  smem_attr_once(done[0], bw::stream_panels_kernel<S, false>, bw::kSmemLimit);
-  smem_attr_once(done[1], bw::stream_panels_kernel<S, true>, bw::kSmemLimit);
+  static bool done[64] = {};
+  smem_attr_once(done, bw::kSmemLimit, bw::stream_panels_kernel<S, false>, bw::stream_panels_kernel<S, true>);
 }
 
 int64_t align256(int64_t v) { return (v + 255) / 256 * 256; }
@@ -811,7 +811,7 @@ int64_t mm_xt_rows(const bw_hmat *h) { return (std::max(h->n_rows, h->n_cols) + 
 void launch_matmat_tc(bw_hmat *h, int o, const double *X, int64_t ldx, double *Y, int64_t ldy, int nrhs, bool permuted,
                       cudaStream_t st) {
   static bool attr_done[64] = {};
-  smem_attr_once(attr_done, bw::mm_stream_kernel, bw::kMmSmem);
+  smem_attr_once(attr_done, bw::kMmSmem, bw::mm_stream_kernel);
   const bw::MmPlan &mm = h->mm[o];
   const int32_t *perm_in = permuted ? nullptr : (o == 0 ? h->d_perm1 : h->d_perm0);
   const int32_t *perm_out = permuted ? nullptr : (o == 0 ? h->d_perm0 : h->d_perm1);
@@ -903,7 +903,7 @@ void launch_multi(bw_hmat *h, int o, int prec, const double *X, int64_t ldx, dou
   using G = typename bw::Store<S>::G;
   using L = bw::MultiLayout<S, K>;
   static bool attr_done[64] = {};
-  smem_attr_once(attr_done, bw::stream_multi_kernel<S, K>, L::kTotal);
+  smem_attr_once(attr_done, L::kTotal, bw::stream_multi_kernel<S, K>);
   const int32_t *perm_in = permuted ? nullptr : (o == 0 ? h->d_perm1 : h->d_perm0);
   const int32_t *perm_out = permuted ? nullptr : (o == 0 ? h->d_perm0 : h->d_perm1);
   const int n_in = (int)h->op[o].n_in;
